@@ -1,5 +1,6 @@
 // gd_fused.cu -- the grid-space part of each nonlinear phase of the
-// mixed-precision step in one kernel: inverse phi transforms of the phase's
+// mixed-precision step in one kernel, for any row length (the lengths of
+// gd_fused_reg.cuh have a register-resident form of the phases with products): inverse phi transforms of the phase's
 // synthesized components, the pointwise products, and the forward phi
 // transform with the Gauss-weighted north/south folds that the Legendre
 // analysis consumes.  The physical grids of a phase live only in shared
@@ -78,10 +79,6 @@ __device__ __forceinline__ void pack_z(float2* bufA, int rs, int n, int e, int r
 // follow from the P-point transforms Y_a of the sub-rows x_(3 c + a):
 //   X_m = sum_a W^(m a) Y_a[m],  X_(n - m) = sum_a W^(-m a) Y_a[(P - m) mod P].
 // Sub-row (pair ii, a) holds P elements at (3 ii + a) P in the xidx layout.
-// The last P-point pass has fewer butterflies than threads, so the split is
-// used where the products are light (the induction phase, the grid output): with the heavier
-// velocity and temperature products the radix-3 pass, which spreads them over
-// every thread, is faster.
 template <int N> struct Split3 {
   static constexpr int P = N / 3;
   static constexpr bool ok = N > 0 && N % 3 == 0 && P >= 8 && (P & (P - 1)) == 0;
@@ -373,30 +370,32 @@ void launch_one_k(cudaStream_t s, const Dims& d, const FftPlan& p, const float2*
   k_fused<N, PH, S3><<<g, FNT, sm, s>>>(d, p, tw, a);
 }
 
-// the three-way split for the induction phase and the grid output whenever
-// the orders fit below n / 3 (the usual dealiased grid nlon = 3 (M + 1))
-template <int N, int PH>
-void launch_one(cudaStream_t s, const Dims& d, const FftPlan& p, const float2* tw, const FusedArgs& a) {
-  if constexpr (Split3<N>::ok && (PH == FUSED_INDUCTION || PH == FUSED_GRID)) {
+// grids on request: the three-way split whenever the orders fit below n / 3
+// (the usual dealiased grid nlon = 3 (M + 1))
+template <int N>
+void launch_grid(cudaStream_t s, const Dims& d, const FftPlan& p, const float2* tw, const FusedArgs& a) {
+  if constexpr (Split3<N>::ok) {
     if (d.M + 1 <= N / 3) {
-      launch_one_k<N, PH, true>(s, d, p, tw, a);
+      launch_one_k<N, FUSED_GRID, true>(s, d, p, tw, a);
       return;
     }
   }
-  launch_one_k<N, PH, false>(s, d, p, tw, a);
-}
-
-template <int N>
-void launch_phase(cudaStream_t s, const Dims& d, const FftPlan& p, const float2* tw, int phase, const FusedArgs& a) {
-  switch (phase) {
-    case FUSED_GRID: launch_one<N, FUSED_GRID>(s, d, p, tw, a); break;
-    case FUSED_TEMPERATURE: launch_one<N, FUSED_TEMPERATURE>(s, d, p, tw, a); break;
-    case FUSED_VELOCITY: launch_one<N, FUSED_VELOCITY>(s, d, p, tw, a); break;
-    default: launch_one<N, FUSED_INDUCTION>(s, d, p, tw, a); break;
-  }
+  launch_one_k<N, FUSED_GRID, false>(s, d, p, tw, a);
 }
 
 }  // namespace
+
+// The phases with products on register-resident transforms (gd_fused_reg.cuh,
+// one file per group of row lengths); fin of the velocity and induction phases
+// in the order theta components, phi components; false (nothing launched) for
+// a length without a row plan.
+bool launch_fused_len1(cudaStream_t s, const Dims& d, int nlon, const void* tw, int phase, const FusedArgs& a);
+bool launch_fused_len2(cudaStream_t s, const Dims& d, int nlon, const void* tw, int phase, const FusedArgs& a);
+bool launch_fused_len3(cudaStream_t s, const Dims& d, int nlon, const void* tw, int phase, const FusedArgs& a);
+bool launch_fused_len4(cudaStream_t s, const Dims& d, int nlon, const void* tw, int phase, const FusedArgs& a);
+bool launch_fused_len5(cudaStream_t s, const Dims& d, int nlon, const void* tw, int phase, const FusedArgs& a);
+bool launch_fused_len6(cudaStream_t s, const Dims& d, int nlon, const void* tw, int phase, const FusedArgs& a);
+bool launch_fused_len7(cudaStream_t s, const Dims& d, int nlon, const void* tw, int phase, const FusedArgs& a);
 
 int fourier_blocks(const Dims& d) { return ceil_div(d.nth, FB); }
 
@@ -406,17 +405,39 @@ size_t fused_smem_bytes(int phase, int nlon) { return fused_smem(phase, nlon, fa
 
 void launch_fused(cudaStream_t s, const Dims& d, const FftPlan& p, const void* twf, int phase, const FusedArgs& a) {
   const float2* tw = static_cast<const float2*>(twf);
-  switch (p.n) {
-    case 24: launch_phase<24>(s, d, p, tw, phase, a); break;
-    case 40: launch_phase<40>(s, d, p, tw, phase, a); break;
-    case 48: launch_phase<48>(s, d, p, tw, phase, a); break;
-    case 96: launch_phase<96>(s, d, p, tw, phase, a); break;
-    case 144: launch_phase<144>(s, d, p, tw, phase, a); break;
-    case 192: launch_phase<192>(s, d, p, tw, phase, a); break;
-    case 288: launch_phase<288>(s, d, p, tw, phase, a); break;
-    case 384: launch_phase<384>(s, d, p, tw, phase, a); break;
-    case 768: launch_phase<768>(s, d, p, tw, phase, a); break;
-    default: launch_phase<0>(s, d, p, tw, phase, a); break;
+  if (phase == FUSED_GRID) {
+    switch (p.n) {
+      case 24: launch_grid<24>(s, d, p, tw, a); break;
+      case 40: launch_grid<40>(s, d, p, tw, a); break;
+      case 48: launch_grid<48>(s, d, p, tw, a); break;
+      case 96: launch_grid<96>(s, d, p, tw, a); break;
+      case 144: launch_grid<144>(s, d, p, tw, a); break;
+      case 192: launch_grid<192>(s, d, p, tw, a); break;
+      case 288: launch_grid<288>(s, d, p, tw, a); break;
+      case 384: launch_grid<384>(s, d, p, tw, a); break;
+      case 768: launch_grid<768>(s, d, p, tw, a); break;
+      default: launch_one_k<0, FUSED_GRID, false>(s, d, p, tw, a); break;
+    }
+    return;
+  }
+  // the products: register-resident rows where the length has a plan, else the
+  // runtime plan (measured at lmax 341, nlon 1024, nr 33 the velocity phase took
+  // 1138 us there and 225 us with a row plan)
+  FusedArgs b = a;
+  if (phase != FUSED_TEMPERATURE)
+    for (int i = 0; i < a.nin / 2; ++i) {
+      b.fin[i] = a.fin[2 * i];
+      b.fin[a.nin / 2 + i] = a.fin[2 * i + 1];
+    }
+  if (launch_fused_len1(s, d, p.n, twf, phase, b) || launch_fused_len2(s, d, p.n, twf, phase, b) ||
+      launch_fused_len3(s, d, p.n, twf, phase, b) || launch_fused_len4(s, d, p.n, twf, phase, b) ||
+      launch_fused_len5(s, d, p.n, twf, phase, b) || launch_fused_len6(s, d, p.n, twf, phase, b) ||
+      launch_fused_len7(s, d, p.n, twf, phase, b))
+    return;
+  switch (phase) {
+    case FUSED_TEMPERATURE: launch_one_k<0, FUSED_TEMPERATURE, false>(s, d, p, tw, a); break;
+    case FUSED_VELOCITY: launch_one_k<0, FUSED_VELOCITY, false>(s, d, p, tw, a); break;
+    default: launch_one_k<0, FUSED_INDUCTION, false>(s, d, p, tw, a); break;
   }
 }
 
