@@ -73,6 +73,15 @@ int build_implicit(gd_handle* h) {
                     h->d_rinv + h->var_rep[v], h->d_rinv2 + h->var_rep[v], h->d_nu, h->c.dt, h->c.implicit_theta,
                     h->c.bc_mode == 2, h->d_lin + h->var_op[v], h->d_lu + h->var_op[v], h->d_flag,
                     h->c.composition ? 4 : 3);
+  auto pack = [&](const double* lu, double2* fac, double* row) {
+    const size_t Lp1 = d.L + 1;
+    for (size_t v = 0; v < h->var_n.size(); ++v)
+      launch_pack_lu(h->stream, h->var_n[v], d.L, h->c.composition ? 4 : 3, h->d_d1 + h->var_band[v],
+                     h->d_d2 + h->var_band[v], h->d_rinv + h->var_rep[v], h->d_rinv2 + h->var_rep[v], h->d_nu,
+                     lu + h->var_op[v], fac + h->var_op[v] / GD_NBW * 5,
+                     row ? row + h->var_op[v] / (GD_NBW * Lp1) * (GD_NBW + 1) : nullptr);
+  };
+  pack(h->d_lu, h->d_fac, h->d_row);
   int s = check_launch(h, "build_lu");
   if (s) return s;
   int flag = 0;
@@ -92,6 +101,8 @@ int build_implicit(gd_handle* h) {
                         h->c.implicit_theta, 1 | (fv << 1), h->d_lu_flux + 3 * h->lu_flux_stride + h->var_op[v],
                         h->d_lu_flux + (size_t)(fv - 1) * h->lu_flux_stride + h->var_op[v], h->d_flag,
                         h->c.composition ? 4 : 3);
+    for (int fv = 1; fv <= 3; ++fv)
+      pack(h->d_lu_flux + (size_t)(fv - 1) * h->lu_flux_stride, h->d_fac + fv * h->fac_stride, nullptr);
     s = check_launch(h, "build_lu (flux rows)");
     if (s) return s;
     CK(cudaMemcpyAsync(&flag, h->d_flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -268,6 +279,9 @@ int setup(gd_handle* h) {
     h->lu_flux_stride = h->var_op.back() + (size_t)4 * h->var_n.back() * nbw * (d.L + 1);
     AL(h->d_lu_flux, 4 * h->lu_flux_stride);
   }
+  h->fac_stride = (h->var_op.back() / nbw + (size_t)4 * h->var_n.back() * (d.L + 1)) * 5;
+  AL(h->d_fac, (c.bc_mode == 2 ? 4 : 1) * h->fac_stride);
+  AL(h->d_row, h->fac_stride / 5 / (d.L + 1) * (nbw + 1));
   AL(h->d_tw, 2 * (size_t)d.nlon); AL(h->d_twf, 2 * (size_t)d.nlon);
   AL(h->d_state, NFIELD * h->spec_elems()); AL(h->d_nl, NFIELD * h->spec_elems());
   AL(h->d_prev, NFIELD * h->spec_elems());
@@ -656,6 +670,10 @@ int implicit_launch(gd_handle* h, int boot) {
   }
   a.lu_flux = h->d_lu_flux;
   a.lu_flux_stride = h->lu_flux_stride;
+  a.fac = h->d_fac;
+  a.fac_flux_stride = h->d_lu_flux ? h->fac_stride : 0;
+  a.fac_bytes = (h->d_lu_flux ? 4 : 1) * h->fac_stride * sizeof(double2);
+  a.row = h->d_row;
   a.inv_dt = 1.0 / h->c.dt;
   a.lin_weight = 1.0 - h->c.implicit_theta;
   a.dt = h->c.dt;

@@ -68,6 +68,10 @@ struct gd_handle {
   double* d_lu_flux = nullptr;
   size_t lu_flux_stride = 0;
   bool flux_rows_ok = false;
+  // the same factors (then the three flux-row sets, fac_stride apart) and the band rows, packed for the step
+  double2* d_fac = nullptr;
+  size_t fac_stride = 0;
+  double* d_row = nullptr;
   // checkpointed forward run of gd_temperature_forward
   std::vector<void*> t_snaps;
   void* t_final = nullptr;

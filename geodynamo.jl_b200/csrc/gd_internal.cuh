@@ -196,7 +196,17 @@ struct Cnab2Args {
   double inv_dt, lin_weight;
   double dt;                  // EAB2: the time step applied to the phi1 term
   int stages;                 // sweeps to run: 1 rhs, 2 forward, 4 back substitution (0: all)
+  // the step's packed operators (launch_pack_lu): factors with, fac_flux_stride
+  // double2 apart, those of the flux rows after them (stride 0: none), and band rows
+  const double2* fac;
+  size_t fac_flux_stride, fac_bytes;
+  const double* row;
+  const double* nu;           // set by launch_cnab2
 };
+// The factors and band rows of launch_build_lu in the step's layout (gd_cnab2.cu);
+// row may be null (factors only).
+void launch_pack_lu(cudaStream_t s, int N, int L, int nkind, const double* d1, const double* d2, const double* rinv,
+                    const double* rinv2, const double* nu, const double* lu, double2* fac, double* row);
 // ---- exponential Adams-Bashforth 2 (gd_expo.cu) ----
 // nkind: 3 (velocity, magnetic, temperature), 4 with composition
 size_t etd_table_doubles(const Dims& d, int nkind);
