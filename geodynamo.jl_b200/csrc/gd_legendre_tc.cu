@@ -68,21 +68,44 @@ __device__ __forceinline__ void put_split_f(float* hi, float* lo, int row, int k
   lo[o] = l;
 }
 
-// 3 TF32 products of one 32-deep chunk into tmem column offset dcol.
+// 3 TF32 products of the first nks 8-deep slices of a chunk into tmem column
+// offset dcol (the slices past the last degree or colatitude hold zeros).
 __device__ __forceinline__ void issue_chunk(uint32_t tmem, uint32_t dcol, const float* Ahi, const float* Alo,
-                                            const float* Bhi, const float* Blo, bool first, uint32_t idesc) {
-  const uint32_t ah = smem_addr(Ahi), al = smem_addr(Alo), bh = smem_addr(Bhi), bl = smem_addr(Blo);
+                                            const float* Bhi, const float* Blo, bool first, uint32_t idesc, int nks) {
+  // descriptors advance by 32 bytes (2 units of 16) per slice of 8 TF32
+  const uint64_t ah = sw128_desc(smem_addr(Ahi)), al = sw128_desc(smem_addr(Alo));
+  const uint64_t bh = sw128_desc(smem_addr(Bhi)), bl = sw128_desc(smem_addr(Blo));
+  tmem += dcol;
 #pragma unroll
   for (int ks = 0; ks < TC_K / 8; ++ks) {
-    const uint32_t off = ks * 32;  // 8 TF32 = 32 bytes along K
-    const uint64_t adh = sw128_desc(ah + off), adl = sw128_desc(al + off);
-    const uint64_t bdh = sw128_desc(bh + off), bdl = sw128_desc(bl + off);
-    mma_tf32(tmem + dcol, adh, bdh, idesc, (first && ks == 0) ? 0u : 1u);
-    mma_tf32(tmem + dcol, adh, bdl, idesc, 1u);
-    mma_tf32(tmem + dcol, adl, bdh, idesc, 1u);
+    if (ks >= nks) break;
+    mma_tf32(tmem, ah + 2 * ks, bh + 2 * ks, idesc, (first && ks == 0) ? 0u : 1u);
+    mma_tf32(tmem, ah + 2 * ks, bl + 2 * ks, idesc, 1u);
+    mma_tf32(tmem, al + 2 * ks, bh + 2 * ks, idesc, 1u);
   }
 }
 
+// D += X0 Y (+ X1 Y, unless null), the slices as above.
+__device__ __forceinline__ void issue_products(uint32_t tmem, const float* X0, const float* X1, const float* Y,
+                                               bool first, uint32_t idesc, int nks) {
+  const uint64_t a0 = sw128_desc(smem_addr(X0)), a1 = sw128_desc(smem_addr(X1 ? X1 : X0)), b = sw128_desc(smem_addr(Y));
+#pragma unroll
+  for (int ks = 0; ks < TC_K / 8; ++ks) {
+    if (ks >= nks) break;
+    mma_tf32(tmem, a0 + 2 * ks, b + 2 * ks, idesc, (first && ks == 0) ? 0u : 1u);
+    if (X1) mma_tf32(tmem, a1 + 2 * ks, b + 2 * ks, idesc, 1u);
+  }
+}
+
+// mbar_wait with one outcome for the whole warp.
+__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int* err, long long limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, limit));
+}
+
+// 8-deep slices with valid degrees in K chunk kc of parity p
+__device__ __forceinline__ int synth_slices(int L, int m, int p, int kc) {
+  return min(TC_K / 8, (kpar(L, m, p) - TC_K * kc + 7) / 8);
+}
 
 }  // namespace
 
@@ -166,29 +189,49 @@ void launch_build_tc_images(cudaStream_t s, const Dims& d, const int* moff, cons
 // ---------------------------------------------------------------------------
 // Synthesis, two kernels.
 //
-// 1. k_synth_coef_image: the runtime coefficients of one call as split,
-//    swizzled TF32 B-operand chunks: chunk (column tile ct, m, step it) =
-//    hi then lo image of NCS columns x 32 K (scalar NCS = 256 columns
-//    n = (field, r, re/im); vector NCS = 128: 32 shells x [S re, S im, T re,
-//    T im]; the valid columns of a tile are a prefix),
+// 1. k_synth_coef_image: the runtime coefficients of one call as swizzled FP32
+//    B-operand chunks: chunk (column tile ct, m, step it) = NCS columns x 32 K
+//    (scalar NCS = 256 columns n = (field, r, re/im); vector NCS = 128: 32 shells
+//    x [S re, S im, T re, T im]; the valid columns of a tile are a prefix),
 //    K -> l = m + p + 2 (32 kc + k).  One CTA per (kc, m, ct) covers both
 //    parities, so each warp reads l-contiguous runs of every coefficient row.
+//    (The radial operators write their chunks themselves.)
 // 2. k_tc_synth4: persistent CTAs over tiles (m, 128-row theta tile, column
-//    tile), 320 threads: warp 0 feeds the two pipeline stages with bulk copies
-//    only (table chunk(s) and the coefficient chunk, transaction bytes on the
-//    stage's `full` barrier), warp 1 issues the split-TF32 MMAs (3 products
-//    per 8-deep K slice) and commits them to the stage's `empty` barrier and,
-//    after a tile's last step, to `tfull`; warps 2-9 (two per TMEM lane
+//    tile), 640 threads.  Warp 0 feeds the slots with bulk copies only (table
+//    chunks, raw coefficient chunk); warps 12-19 split a raw chunk to TF32 hi /
+//    lo at the same swizzled offsets; warps 1 and 2 issue the split-TF32 MMAs
+//    (3 products per 8-deep K slice holding degrees) of the even and the odd
+//    parity, whose accumulators are disjoint; warps 4-11 (two per TMEM lane
 //    quarter, alternate 8-column chunks) wait on `tfull`, read the
 //    accumulators, release them on `tempty` and write the blocked Fourier
-//    layout while the next tile's stages are already loading.  Scalar: accumulators [even | odd] x 256.
-//    Vector: [P even | P odd | dP even | dP odd] x 128; the m/sin(theta) of
-//    the Q = m Pbar / sin(theta) terms is applied to the Pbar sums.  Rows past
-//    the last colatitude and columns past the last shell are neither copied
-//    nor (columns) multiplied: the MMA width follows the tile's valid columns.
+//    layout while the next tile's slots are already filling.  Scalar:
+//    accumulators [even | odd] x 256.  Vector: [P even | P odd | dP even |
+//    dP odd] x 128; the m/sin(theta) of the Q = m Pbar / sin(theta) terms is
+//    applied to the Pbar sums.  Rows past the last colatitude and columns past
+//    the last shell are neither copied nor (columns) multiplied: the MMA width
+//    follows the tile's valid columns.
+// What bounds it (lmax 255, nr 129, vector, 152 us): the MMAs alone take 60 us
+// (N = 128 issues every 64 clocks, N = 256 every 128), issue bookkeeping and the
+// hand-over of the accumulators between tiles another 40, the copies and the
+// stores (which the hand-over does not hide) the rest; without MMAs it runs in
+// 109 us.  Chunks that cross memory as FP32 instead of hi and lo halve what the
+// pre-pass and the radial operators write: pre-pass 54 -> 36 us, curl 100 -> 84,
+// gradients 142 -> 98; the synthesis itself at lmax 341, nr 33: 153 -> 137 us
+// (vector), lmax 127, nr 65: 33 -> 30, 53 -> 46 (scalar).
 // ---------------------------------------------------------------------------
-constexpr int SY_THREADS = 320;  // producer, MMA issuer, 8 epilogue warps (two per TMEM lane quarter)
-constexpr int SY_EPI = SY_THREADS - 64;
+// Shared memory: 32 KB slots for the operand that both halves of a step use
+// (vector three: the coefficient chunk, hi and lo; scalar two: the table chunk) and
+// a ring of four 32 KB slots for the halves (vector: Pbar chunk, dPbar chunk;
+// scalar: coefficient hi image, lo image), each with its own full / empty barriers.
+// A raw chunk lands where its hi image will be and is split in place.
+// An issuer sees every other step, so the barrier phase it waits for must not be
+// two ahead of the slot's: slots filled by bulk copies, which may land in any
+// order, are even in number (within a tile one issuer's own); the three are filled
+// by the converters, in step order, so a step that is full has all earlier ones full.
+constexpr int SY_THREADS = 640;
+constexpr int SY_EPI_WARPS = 8, SY_CONV_WARPS = 8;
+constexpr int SY_HMAX = 3, SY_S = 4;
+constexpr int SY_SLOT = CHUNK_FLOATS;  // floats
 
 // step it -> (parity p, K chunk kc): odd-parity chunks interleave with the
 // even ones while both exist
@@ -233,8 +276,8 @@ __global__ void __launch_bounds__(256) k_synth_coef_image(Dims d, const int* __r
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long base = (long)ct * a.ttot + cofs[m] / ntt;
-  float* h0 = a.bimg + (base + synth_step_of(0, kc, nc1)) * (2L * BT);
-  float* h1 = kc < nc1 ? a.bimg + (base + synth_step_of(1, kc, nc1)) * (2L * BT) : nullptr;
+  float* h0 = a.bimg + (base + synth_step_of(0, kc, nc1)) * (long)BT;
+  float* h1 = kc < nc1 ? a.bimg + (base + synth_step_of(1, kc, nc1)) * (long)BT : nullptr;
   const int l0 = m + 2 * (TC_K * kc + lane);
   // rows in batches of four per warp, every load of a batch issued before its stores
   constexpr int RB = 4;
@@ -253,14 +296,8 @@ __global__ void __launch_bounds__(256) k_synth_coef_image(Dims d, const int* __r
       // rows of other fields are written by their producer kernels
       if (row < NCS && mine[row]) {
         const uint32_t o = sw128_offset(row, lane) >> 2;
-        const float f0 = __double2float_rn(v0[u]), g0 = tf32_rn(f0);
-        h0[o] = g0;
-        h0[BT + o] = tf32_rn(f0 - g0);
-        if (h1 != nullptr) {
-          const float f1 = __double2float_rn(v1[u]), g1 = tf32_rn(f1);
-          h1[o] = g1;
-          h1[BT + o] = tf32_rn(f1 - g1);
-        }
+        h0[o] = __double2float_rn(v0[u]);
+        if (h1 != nullptr) h1[o] = __double2float_rn(v1[u]);
       }
     }
   }
@@ -273,18 +310,22 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
                                                              const float* __restrict__ imgD,
                                                              const double* __restrict__ sinv, TcSynthArgs a, int ntt,
                                                              int ncol) {
-  constexpr int S = 2;
   constexpr int NCS = VEC ? TC_N2 : 2 * TC_N2;   // columns per tile: vector 128, scalar 256
-  constexpr int A_FL = (VEC ? 2 : 1) * CHUNK_FLOATS;
   constexpr int BT = NCS * TC_K;                  // one B image (hi or lo)
-  constexpr int ST_FL = A_FL + 2 * BT;
   constexpr uint32_t NCOL = 512;
   extern __shared__ unsigned char smem_raw[];
   const uintptr_t base = (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023);
-  float* stg = reinterpret_cast<float*>(base);
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + (size_t)S * ST_FL * 4);
-  uint64_t* empty = full + S;
-  uint64_t* tfull = empty + S;
+  constexpr int SY_H = VEC ? 3 : 2;
+  constexpr int SY_R = VEC ? SY_H : SY_S / 2;          // coefficient chunks
+  static_assert(SY_S % 2 == 0 && (VEC || SY_H % 2 == 0) && SY_H <= SY_HMAX, "slots");
+  float* const hst = reinterpret_cast<float*>(base);   // SY_H slots
+  float* const sst = hst + SY_H * SY_SLOT;             // SY_S slots
+  uint64_t* hfull = reinterpret_cast<uint64_t*>(base + (size_t)(SY_H + SY_S) * SY_SLOT * 4);
+  uint64_t* hempty = hfull + SY_H;
+  uint64_t* sfull = hempty + SY_H;
+  uint64_t* sempty = sfull + SY_S;
+  uint64_t* rfull = sempty + SY_S;  // raw coefficient chunk landed
+  uint64_t* tfull = rfull + SY_H;
   uint64_t* tempty = tfull + 1;
   uint64_t* drain = tempty + 1;  // after a failed wait: completion of the MMAs already issued
   uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 1);
@@ -293,13 +334,19 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
   const int Ntot = a.nf * d.nr * 2;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
+    // the split operand's slots are filled by the converter warps, the table's by bulk copies
+    for (int s = 0; s < SY_H; ++s) {
+      mbar_init(&hfull[s], VEC ? SY_CONV_WARPS : 1);
+      mbar_init(&hempty[s], 1);
     }
-    mbar_init(tfull, 1);
-    mbar_init(tempty, SY_EPI);
-    mbar_init(drain, 1);
+    for (int s = 0; s < SY_S; ++s) {
+      mbar_init(&sfull[s], VEC ? 1 : SY_CONV_WARPS);
+      mbar_init(&sempty[s], 1);
+    }
+    for (int s = 0; s < SY_R; ++s) mbar_init(&rfull[s], 1);
+    mbar_init(tfull, 2);  // one commit per MMA issuer
+    mbar_init(tempty, SY_EPI_WARPS);  // one arrival per epilogue warp
+    mbar_init(drain, 2);
   }
   if (warp == 0) tmem_alloc(tslot, NCOL);
   fence_before_sync();
@@ -308,7 +355,9 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
   const uint32_t tmem = *tslot;
   const int ntiles = (d.M + 1) * ntt * ncol;
   bool ok = true;
-  int issued = -1;  // producer: last pipeline step whose bulk copies were issued
+  // producer: phase of each slot's last issued copies (-1: none): tables (vector: the
+  // ring, scalar: the shared slots) and raw chunks
+  int tlast[SY_S] = {-1, -1, -1, -1}, rlast[SY_HMAX] = {-1, -1, -1};
 
   if (warp == 0) {
     // producer: bulk copies only.  Step (tile tt, it): table chunk(s) and the
@@ -316,93 +365,154 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
     // columns past the last valid one only reach accumulator rows / columns
     // the epilogue never reads, so whole 8-row swizzle atoms of the rest are
     // copied.
-    auto step_src = [&](int tt, int it, const float*& s0, const float*& s1, const float*& sb, uint32_t& pa,
-                        uint32_t& pb) {
-      const int m = tt / (ntt * ncol), tile = (tt / ncol) % ntt, ct = tt % ncol;
-      const int nc1 = nck_h(L, m, 1);
-      int p, kc;
-      synth_step_pk(it, nc1, p, kc);
-      const long ch = synth_chunk(cofs, L, m, tile, p, kc);
-      const long bch = (long)ct * a.ttot + cofs[m] / ntt + it;
-      pa = (uint32_t)min(TC_M, (d.nth - tile * TC_M + 7) & ~7) * 128u;
-      const int nvalid = VEC ? 4 * min(32, d.nr - ct * 32) : min(NCS, Ntot - ct * NCS);
-      pb = (uint32_t)((nvalid + 7) & ~7) * 128u;
-      s0 = imgP + ch * CHUNK_FLOATS;
-      s1 = imgD + ch * CHUNK_FLOATS;
-      sb = a.bimg + bch * (2L * BT);
-    };
     int gs = 0;
     for (int tt = blockIdx.x; tt < ntiles && ok; tt += gridDim.x) {
-      const int m = tt / (ntt * ncol);
+      const int m = tt / (ntt * ncol), tile = (tt / ncol) % ntt, ct = tt % ncol;
       const int nc1 = nck_h(L, m, 1), T = nck_h(L, m, 0) + nc1;
-      for (int it = 0; it < T; ++it) {
-        const int G = gs + it, s = G & 1, u = G >> 1;
-        if (u >= 1 && !mbar_wait(&empty[s], (u - 1) & 1, a.err, a.wait_limit)) {
+      const uint32_t pa = (uint32_t)min(TC_M, (d.nth - tile * TC_M + 7) & ~7) * 128u;
+      const int nvalid = VEC ? 4 * min(32, d.nr - ct * 32) : min(NCS, Ntot - ct * NCS);
+      const uint32_t pb = (uint32_t)((nvalid + 7) & ~7) * 128u;
+      const float* const bsrc = a.bimg + ((long)ct * a.ttot + cofs[m] / ntt) * (long)BT;
+      for (int it = 0; it < T && ok; ++it) {
+        const int G = gs + it;
+        int p, kc;
+        synth_step_pk(it, nc1, p, kc);
+        const long ch = synth_chunk(cofs, L, m, tile, p, kc) * CHUNK_FLOATS;
+        // error-path tests: CTA 0 may omit one step's copies, so the bounded
+        // waits on its slots run out
+        const bool omit = a.omit_plus1 == G + 1 && blockIdx.x == 0;
+        const int rs = G % SY_R, ru = G / SY_R;
+        // the chunk's slots: vector one of the shared ones, scalar a hi / lo pair of the ring
+        if (ru >= 1 && !(VEC ? wait_all(&hempty[rs], (ru - 1) & 1, a.err, a.wait_limit)
+                             : wait_all(&sempty[2 * rs], (ru - 1) & 1, a.err, a.wait_limit) &&
+                                   wait_all(&sempty[2 * rs + 1], (ru - 1) & 1, a.err, a.wait_limit))) {
           ok = false;
           break;
         }
-        // error-path tests: CTA 0 may omit one step's copies, so the MMA
-        // warp's bounded wait on that stage runs out
-        const bool omit = a.omit_plus1 == G + 1 && blockIdx.x == 0;
-        if (lane == 0 && !omit) {
-          float* A = stg + s * ST_FL;
-          const float *s0, *s1, *sb;
-          uint32_t pa, pb;
-          step_src(tt, it, s0, s1, sb, pa, pb);
-          mbar_arrive_expect_tx(&full[s], (VEC ? 4u : 2u) * pa + 2u * pb);
-          bulk_g2s(A, s0, pa, &full[s]);
-          bulk_g2s(A + TILE_A_FLOATS, s0 + TILE_A_FLOATS, pa, &full[s]);
-          if (VEC) {
-            bulk_g2s(A + CHUNK_FLOATS, s1, pa, &full[s]);
-            bulk_g2s(A + CHUNK_FLOATS + TILE_A_FLOATS, s1 + TILE_A_FLOATS, pa, &full[s]);
+        if (!omit) {
+          if (lane == 0) {
+            mbar_arrive_expect_tx(&rfull[rs], pb);
+            bulk_g2s(VEC ? hst + rs * SY_SLOT : sst + 2 * rs * SY_SLOT, bsrc + (long)it * BT, pb, &rfull[rs]);
           }
-          bulk_g2s(A + A_FL, sb, pb, &full[s]);
-          bulk_g2s(A + A_FL + BT, sb + BT, pb, &full[s]);
+#pragma unroll
+          for (int q = 0; q < SY_R; ++q) rlast[q] = rs == q ? ru : rlast[q];
         }
-        if (!omit) issued = G;
+#pragma unroll
+        for (int x = 0; x < (VEC ? 2 : 1); ++x) {
+          const int Q = VEC ? 2 * G + x : G, NS = VEC ? SY_S : SY_H, qs = Q % NS, qu = Q / NS;
+          uint64_t* const fullb = VEC ? &sfull[qs] : &hfull[qs];
+          if (qu >= 1 && !wait_all(VEC ? &sempty[qs] : &hempty[qs], (qu - 1) & 1, a.err, a.wait_limit)) {
+            ok = false;
+            break;
+          }
+          if (omit) continue;
+          if (lane == 0) {
+            float* D = (VEC ? sst : hst) + qs * SY_SLOT;
+            const float* s0 = (x == 0 ? imgP : imgD) + ch;
+            mbar_arrive_expect_tx(fullb, 2u * pa);
+            bulk_g2s(D, s0, pa, fullb);
+            bulk_g2s(D + TILE_A_FLOATS, s0 + TILE_A_FLOATS, pa, fullb);
+          }
+#pragma unroll
+          for (int q = 0; q < SY_S; ++q) tlast[q] = qs == q ? qu : tlast[q];
+        }
         __syncwarp();
       }
       gs += T;
     }
-  } else if (warp == 1) {
-    // MMA issuer
+  } else if (warp >= 12) {
+    // converters: x = hi + lo, hi = tf32(x), lo = tf32(x - hi), element by element
+    int gs = 0;
+    for (int tt = blockIdx.x; tt < ntiles && ok; tt += gridDim.x) {
+      const int m = tt / (ntt * ncol), ct = tt % ncol;
+      const int T = nck_h(L, m, 0) + nck_h(L, m, 1);
+      const int nvalid = VEC ? 4 * min(32, d.nr - ct * 32) : min(NCS, Ntot - ct * NCS);
+      const int n4 = ((nvalid + 7) & ~7) * (TC_K / 4);
+      for (int it = 0; it < T && ok; ++it) {
+        const int G = gs + it, rs = G % SY_R;
+        if (!wait_all(&rfull[rs], (G / SY_R) & 1, a.err, a.wait_limit)) {
+          ok = false;
+          break;
+        }
+        float* const hi = VEC ? hst + rs * SY_SLOT : sst + 2 * rs * SY_SLOT;
+        float* const lo = hi + (VEC ? TILE_A_FLOATS : SY_SLOT);
+        for (int e = tid - 12 * 32; e < n4; e += 32 * SY_CONV_WARPS) {
+          const float4 v = reinterpret_cast<const float4*>(hi)[e];
+          float4 h, l;
+          h.x = tf32_rn(v.x); h.y = tf32_rn(v.y); h.z = tf32_rn(v.z); h.w = tf32_rn(v.w);
+          l.x = tf32_rn(v.x - h.x); l.y = tf32_rn(v.y - h.y); l.z = tf32_rn(v.z - h.z); l.w = tf32_rn(v.w - h.w);
+          reinterpret_cast<float4*>(hi)[e] = h;
+          reinterpret_cast<float4*>(lo)[e] = l;
+        }
+        fence_proxy_async();  // the MMAs read through the async proxy
+        __syncwarp();
+        if (lane == 0) {
+          if (VEC) {
+            mbar_arrive(&hfull[rs]);
+          } else {
+            mbar_arrive(&sfull[2 * rs]);
+            mbar_arrive(&sfull[2 * rs + 1]);
+          }
+        }
+      }
+      gs += T;
+    }
+  } else if (warp <= 2) {
+    // MMA issuers: warp 1 the even, warp 2 the odd parity, whose accumulators
+    // are disjoint.  A step's ~20 instructions take 64 clocks each, and the one
+    // warp's own bookkeeping (waits, addresses) about 1100 clocks a step, during
+    // which the tensor core ran dry; with two, one issues while the other waits.
+    const int p = warp - 1;
     int gs = 0, q = 0;
     for (int tt = blockIdx.x; tt < ntiles && ok; tt += gridDim.x, ++q) {
       const int m = tt / (ntt * ncol), ct = tt % ncol;
-      const int nc1 = nck_h(L, m, 1), T = nck_h(L, m, 0) + nc1;
+      const int nc1 = nck_h(L, m, 1), nc0 = nck_h(L, m, 0), T = nc0 + nc1;
       const int nvalid = VEC ? 4 * min(32, d.nr - ct * 32) : min(NCS, Ntot - ct * NCS);
       const uint32_t ids = idesc_tf32(TC_M, (nvalid + 15) & ~15);
-      if (q >= 1 && !mbar_wait(tempty, (q - 1) & 1, a.err, a.wait_limit)) {
+      const int nc = p == 0 ? nc0 : nc1;
+      if (q >= 1 && !wait_all(tempty, (q - 1) & 1, a.err, a.wait_limit)) {
         ok = false;
         break;
       }
-      for (int it = 0; it < T; ++it) {
-        const int G = gs + it, s = G & 1;
-        if (!mbar_wait(&full[s], (G >> 1) & 1, a.err, a.wait_limit)) {
+      for (int kc = 0; kc < nc && ok; ++kc) {
+        const int G = gs + synth_step_of(p, kc, nc1), hs = G % SY_H;
+        const int nks = synth_slices(L, m, p, kc);
+        const float* H = hst + hs * SY_SLOT;
+        if (!wait_all(&hfull[hs], (G / SY_H) & 1, a.err, a.wait_limit)) {
           ok = false;
           break;
         }
-        fence_after_sync();
-        if (lane == 0) {
-          int p, kc;
-          synth_step_pk(it, nc1, p, kc);
-          const float* A = stg + s * ST_FL;
-          const float* B = A + A_FL;
 #pragma unroll
-          for (int t = 0; t < (VEC ? 2 : 1); ++t)
-            issue_chunk(tmem, (t * 2 + p) * NCS, A + t * CHUNK_FLOATS, A + t * CHUNK_FLOATS + TILE_A_FLOATS, B,
-                        B + BT, kc == 0, ids);
-          mma_commit(smem_addr(&empty[s]));
-          if (it == T - 1) mma_commit(smem_addr(tfull));
+        for (int x = 0; x < 2; ++x) {
+          const int Q = 2 * G + x, qs = Q % SY_S;
+          if (!wait_all(&sfull[qs], (Q / SY_S) & 1, a.err, a.wait_limit)) {
+            ok = false;
+            break;
+          }
+          fence_after_sync();
+          if (elect_one()) {
+            const float* D = sst + qs * SY_SLOT;
+            if (VEC) {
+              issue_chunk(tmem, (x * 2 + p) * NCS, D, D + TILE_A_FLOATS, H, H + TILE_A_FLOATS, kc == 0, ids, nks);
+            } else {  // coefficient hi image with both table images, lo image with the hi table
+              issue_products(tmem + p * NCS, H, x == 0 ? H + TILE_A_FLOATS : nullptr, D, kc == 0 && x == 0, ids, nks);
+            }
+            mma_commit(smem_addr(&sempty[qs]));
+            if (x == 1) {
+              mma_commit(smem_addr(&hempty[hs]));
+              if (kc == nc - 1) mma_commit(smem_addr(tfull));
+            }
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
+      if (nc == 0 && lane == 0) mbar_arrive(tfull);  // an order without odd degrees
       gs += T;
     }
-  } else {
-    // epilogue warps 2-9: TMEM lane quarter warp & 3; the two warps of a
+  } else if (warp >= 4) {
+    // epilogue warps 4-11: TMEM lane quarter warp & 3; the two warps of a
     // quarter take alternate 8-column chunks
-    const int qw = warp & 3, half = (warp - 2) >> 2;
+    const int qw = warp & 3, half = (warp - 4) >> 2;
     // scalar columns n = (f nr + r) 2 + re/im: the pair n / 2 = f nr + r indexes the (comp, r) run
     const size_t run = (size_t)a.nblk * (d.M + 1) * FOURIER_BLOCK;
     const uint32_t trow = tmem + ((uint32_t)(qw * 32) << 16);
@@ -425,7 +535,8 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
       const int clast = mine > 0 ? 8 * (half + 2 * (mine - 1)) : -1;
       if (clast < 0) {
         fence_before_sync();
-        mbar_arrive(tempty);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty);
       }
       if (!VEC) {
         for (int c0 = 8 * half; c0 < cend; c0 += 16) {
@@ -439,7 +550,8 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
           }
           if (c0 == clast) {
             fence_before_sync();
-            mbar_arrive(tempty);  // accumulators read: the next tile's MMAs may start
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty);  // accumulators read: the next tile's MMAs may start
           }
           if (ith < d.nth) {
 #pragma unroll
@@ -470,7 +582,8 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
           }
           if (c0 == clast) {
             fence_before_sync();
-            mbar_arrive(tempty);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty);
           }
           if (ith < d.nth) {
 #pragma unroll
@@ -505,12 +618,19 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
     }
   }
   ok = __syncthreads_and(ok);
-  // after an expired wait anywhere in the CTA: the producer lets its last bulk
-  // copies land (a step the MMA warp consumed has completed its phase
-  // already, so this returns at once), and the MMA warp waits for the MMAs it
-  // has issued, before tensor memory is freed and the CTA exits
-  if (!ok && warp == 0 && issued >= 0) mbar_wait(&full[issued & 1], (issued >> 1) & 1, a.err, a.wait_limit);
-  if (!ok && warp == 1) {
+  // after an expired wait anywhere in the CTA: the producer lets the copies it
+  // issued last on every slot land (a phase already complete returns at once),
+  // and the MMA warp waits for the MMAs it has issued, before tensor memory is
+  // freed and the CTA exits
+  if (!ok && warp == 0) {
+#pragma unroll
+    for (int s = 0; s < (VEC ? SY_S : SY_H); ++s)
+      if (tlast[s] >= 0) mbar_wait(VEC ? &sfull[s] : &hfull[s], tlast[s] & 1, a.err, a.wait_limit);
+#pragma unroll
+    for (int s = 0; s < SY_R; ++s)
+      if (rlast[s] >= 0) mbar_wait(&rfull[s], rlast[s] & 1, a.err, a.wait_limit);
+  }
+  if (!ok && (warp == 1 || warp == 2)) {
     if (lane == 0) mma_commit(smem_addr(drain));
     __syncwarp();
     mbar_wait(drain, 0, a.err, a.wait_limit);
@@ -702,16 +822,18 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_analysis3(Dims d, const in
         break;
       }
       fence_after_sync();
-      if (lane == 0) {
+      __syncwarp();
+      if (elect_one()) {
         const int cc = it / ns, p = it % ns;
+        const int nks = min(TC_K / 8, (d.nth - TC_K * cc + 7) / 8);
         const float* A = stg + s * ST_FL;
         const float* B = A + A_FL;
         if (!VEC) {
-          issue_chunk(tmem, p * NC, A, A + TILE_A_FLOATS, B, B + BT, cc == 0, idesc);
+          issue_chunk(tmem, p * NC, A, A + TILE_A_FLOATS, B, B + BT, cc == 0, idesc, nks);
         } else {  // fold p: dPbar rows of parity 1 - p, Q rows of parity p
-          issue_chunk(tmem, (0 * 2 + 1 - p) * NC, A, A + TILE_A_FLOATS, B, B + BT, cc == 0, idesc);
+          issue_chunk(tmem, (0 * 2 + 1 - p) * NC, A, A + TILE_A_FLOATS, B, B + BT, cc == 0, idesc, nks);
           issue_chunk(tmem, (1 * 2 + p) * NC, A + CHUNK_FLOATS, A + CHUNK_FLOATS + TILE_A_FLOATS, B, B + BT,
-                      cc == 0, idesc);
+                      cc == 0, idesc, nks);
         }
         mma_commit(smem_addr(&empty[s]));
       }
@@ -806,8 +928,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_analysis3(Dims d, const in
 // address slot and the scalar kernels' per-column tables (one pointer per
 // column, one offset per pair).
 static size_t synth_smem(bool vec) {
-  const int S = 2, NCS = vec ? TC_N2 : 2 * TC_N2, A = (vec ? 2 : 1) * CHUNK_FLOATS, B = 2 * NCS * TC_K;
-  return 1024 + (size_t)S * (A + B) * 4 + 8 * (2 * S + 4);
+  (void)vec;
+  return 1024 + (size_t)(SY_HMAX + SY_S) * SY_SLOT * 4 + 8 * (3 * SY_HMAX + 2 * SY_S + 4);
 }
 static size_t analysis_smem(bool vec) {
   const int S = 2, NC = TC_N2, A = (vec ? 2 : 1) * CHUNK_FLOATS;
@@ -849,7 +971,7 @@ void launch_tc_synth(cudaStream_t s, const Dims& d, const int* moff, const long*
 
 size_t tc_synth_bimage_floats(const Dims& d, long ttot) {
   const long ncol_s = ceil_div(4L * d.nr * 2, 2 * TC_N2), ncol_v = ceil_div(d.nr, 32);
-  const long s = ncol_s * ttot * 2L * (2 * TC_N2) * TC_K, v = ncol_v * ttot * 2L * TC_N2 * TC_K;
+  const long s = ncol_s * ttot * (2L * TC_N2) * TC_K, v = ncol_v * ttot * (long)TC_N2 * TC_K;
   return (size_t)(s > v ? s : v);
 }
 

@@ -37,7 +37,7 @@ struct MixedState {
   float4* d_Fall = nullptr;    // FC_COUNT blocked components
   size_t fcomp = 0;            // float4 per component
   float2* d_G = nullptr;       // folded transforms for the analysis, 2 components
-  // split coefficient images of the synthesis (zeroed once; every writer
+  // coefficient images of the synthesis (zeroed once; every writer
   // keeps its layout's padding at zero): scalar (T by the pre-pass, its
   // gradient by k_gradients), vector state fields (pre-pass), vector curls (k_curl)
   float* d_bimg_s = nullptr;

@@ -18,8 +18,8 @@ __host__ __device__ __forceinline__ int tc_nck(int L, int m, int p) {
 __host__ __device__ __forceinline__ int tc_step_of(int p, int kc, int nc1) { return kc < nc1 ? 2 * kc + p : nc1 + kc; }
 
 // Destination of runtime coefficients written straight into a synthesis
-// B image (split TF32 hi / lo, 128-byte swizzled): chunk (column tile ct, m,
-// step) at ct * ttot + bofs[m] + step, NCS columns x 32 K each.
+// B image (FP32, 128-byte swizzled; the synthesis splits it to TF32 hi / lo):
+// chunk (column tile ct, m, step) at ct * ttot + bofs[m] + step, NCS columns x 32 K each.
 struct SynthImageOut {
   float* img;         // null: write FP64 outputs instead
   const long* bofs;   // first step of order m within a column tile
@@ -37,14 +37,11 @@ __device__ __forceinline__ SynthImagePos synth_image_pos(const SynthImageOut& o,
   const int q = l - m, p = q & 1, idx = q >> 1;
   return SynthImagePos{o.bofs[m] + tc_step_of(p, idx >> 5, tc_nck(L, m, 1)), idx & 31};
 }
-// Split v = hi + lo into column col of column tile ct.
+// v into column col of column tile ct.
 __device__ __forceinline__ void synth_image_put(const SynthImageOut& o, int ncs, const SynthImagePos& at, int ct,
                                                 int col, double v) {
-  float* hi = o.img + ((long)ct * o.ttot + at.step) * (2L * ncs * 32);
-  const uint32_t off = tc::sw128_offset((uint32_t)col, (uint32_t)at.k) >> 2;
-  const float f = __double2float_rn(v), h = tc::tf32_rn(f);
-  hi[off] = h;
-  hi[(size_t)ncs * 32 + off] = tc::tf32_rn(f - h);
+  float* chunk = o.img + ((long)ct * o.ttot + at.step) * (ncs * 32L);
+  chunk[tc::sw128_offset((uint32_t)col, (uint32_t)at.k) >> 2] = __double2float_rn(v);
 }
 
 // Colatitude pairs per block of the blocked Fourier layout written by the
@@ -60,7 +57,7 @@ struct TcSynthArgs {
   int* err;               // set to 1 if a bounded wait expires
   long long wait_limit;   // clock cycles of each bounded wait (0: the default)
   int omit_plus1;         // > 0: CTA 0 omits the bulk copies of pipeline step omit_plus1 - 1 (error-path tests)
-  float* bimg;            // split coefficient images (tc_synth_bimage_floats floats)
+  float* bimg;            // coefficient images (tc_synth_bimage_floats floats)
   long ttot;              // pipeline steps summed over m (one column tile)
   int prep_mask;          // fields the pre-pass writes into bimg (the others are written by their producer)
   int max_ctas;           // persistent CTAs of the launch (0: one per SM)

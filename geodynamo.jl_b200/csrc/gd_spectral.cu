@@ -74,7 +74,7 @@ static size_t radial_smem() {
 // theta derivative by the reference's recurrence coefficients (:158,171), phi
 // derivative i m, radial derivative by the banded D1, then x 1/r on the
 // angular components (:317-321).  In m-major order (l +- 1, m) sits at j +- 1.
-// IMG: the mixed path's scalar synthesis reads g_theta, g_phi, g_r as split
+// IMG: the mixed path's scalar synthesis reads g_theta, g_phi, g_r as
 // TF32 image columns (field slots 1, 2, 3 of n = (field nr + r) 2 + re/im);
 // they are written there instead of to the FP64 arrays.
 template <int KL, bool IMG>
@@ -186,7 +186,7 @@ void launch_gradients_img(cudaStream_t s, const Dims& d, const int* lof, const i
 // compute_vorticity_spectral_full! (src/velocity.jl:340-441) and
 // compute_current_density_spectral! (src/magnetic.jl:253-349):
 //   curl_tor = l(l+1)/r^2 P - D2 P - (2/r) D1 P,   curl_pol = -l(l+1)/r^2 T.
-// IMG: the mixed path's vector synthesis of the curl reads it as split TF32
+// IMG: the mixed path's vector synthesis of the curl reads it as FP32
 // image columns 32 shells x [S re, S im, T re, T im] (S = curl_pol, T =
 // curl_tor), column tile r / 32; written there instead of to the FP64 arrays.
 template <int KL, bool IMG>

@@ -44,6 +44,15 @@ __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// One lane of a converged warp.  A branch on it (unlike lane == 0) leaves the
+// operands of the tensor-core instructions in uniform registers, where they
+// are read from; they were moved there one by one for every instruction.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
@@ -122,9 +131,7 @@ constexpr long long kWaitCycles = 1LL << 31;
 // false then.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, long long limit = 0) {
   const uint32_t addr = smem_addr(bar);
-  const long long bound = limit > 0 ? limit : kWaitCycles;
-  const long long t0 = clock64();
-  while (true) {
+  auto test = [&] {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -133,7 +140,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
         : "=r"(done)
         : "r"(addr), "r"(parity)
         : "memory");
-    if (done) return true;
+    return done != 0;
+  };
+  if (test()) return true;  // without reading the clock
+  const long long bound = limit > 0 ? limit : kWaitCycles;
+  const long long t0 = clock64();
+  while (true) {
+    if (test()) return true;
     if (clock64() - t0 > bound) {
       atomicExch(err, 1);
       return false;
