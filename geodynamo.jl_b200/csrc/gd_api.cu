@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -20,6 +21,10 @@ namespace {
 
 // State fields of the configuration: the five of the reference's step, and
 // composition when configured.
+// Largest four-component Fourier buffer of a model whose captured step runs its
+// phases side by side (step_sequence_forked); above, the kernels fill the chip.
+constexpr size_t FORK_BYTES = (size_t)64 << 20;
+
 int nfields(const gd_handle* h) { return h->c.composition ? NFIELD : NFIELD - 1; }
 
 int fail(gd_handle* h, int code, const std::string& msg) {
@@ -290,7 +295,13 @@ int setup(gd_handle* h) {
   AL(h->d_cbvals, 2 * NL); AL(h->d_csources, NR); AL(h->d_bctype, 4 * NL); AL(h->d_tau, 4 * NR);
   AL(h->d_tauc, 6 * (size_t)d.nseg);
   AL(h->d_grid, NGRID * h->grid_elems());
-  AL(h->d_F, (size_t)4 * NR * (d.M + 1) * d.nlat);
+  {
+    // with room for the phases of a captured step side by side where they run so
+    const size_t comp = NR * (d.M + 1) * d.nlat;
+    const bool more = c.precision == GD_PREC_FP64 && c.magnetic && !c.composition && 4 * comp * sizeof(double2) <= FORK_BYTES;
+    AL(h->d_F, (more ? 12 : 4) * comp);
+    if (more) h->d_F2 = h->d_F + 4 * comp;
+  }
   AL(h->d_epart, 2 * GD_ENERGY_BLOCKS * d.nseg); AL(h->d_eout, 2 * d.nseg);
 
   cudaStream_t s = h->stream;
@@ -753,6 +764,131 @@ int step_sequence(gd_handle* h, int boot) {
   return implicit_launch(h, boot);
 }
 
+// The same step for a captured graph of a small FP64 model, its phases side by
+// side: a step there is a chain of about twenty kernels of 5-10 us that leave
+// most of the chip idle.  What a phase reads of another orders them: the
+// temperature products read the velocity grids of the step before, so the new
+// ones are written after them; the velocity products read j and B of the step
+// before, the induction the new velocity.  The kernels and their inputs are those
+// of step_sequence, so are the results, to the last bit.
+// Measured (B200, us a step, chain -> side by side): lmax 31, nr 32 CNAB2: 155 ->
+// 99; lmax 63, nr 65 EAB2, with loading and reading the state: 463 -> 396.
+bool can_fork(const gd_handle* h) {
+  const size_t comp = (size_t)h->d.nr * (h->d.M + 1) * h->d.nlat * sizeof(double2);
+  return h->precision == GD_PREC_FP64 && !h->ext_derivs && h->c.magnetic && !h->c.composition && 4 * comp <= FORK_BYTES;
+}
+
+// Two streams per device that carry the branches while a step is captured (the
+// graph keeps none of them): made once, held by one capture at a time.
+struct ForkStreams {
+  std::mutex mu;
+  cudaStream_t s[2] = {nullptr, nullptr};
+};
+ForkStreams* fork_streams(int device) {
+  static ForkStreams pool[64];
+  if (device < 0 || device >= 64) return nullptr;
+  ForkStreams* f = &pool[device];
+  std::lock_guard<std::mutex> lock(f->mu);
+  for (auto& s : f->s)
+    if (!s && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+      s = nullptr;
+      cudaGetLastError();
+      return nullptr;
+    }
+  return f;
+}
+
+int step_sequence_forked(gd_handle* h, int boot, const cudaStream_t* fork) {
+  const Dims& d = h->d;
+  const cudaStream_t s0 = h->stream, s1 = fork[0], s2 = fork[1];
+  const size_t comp = (size_t)d.nr * (d.M + 1) * d.nlat, G = h->grid_elems();
+  double2 *const Fv = h->d_F2, *const Fm = h->d_F2 + 4 * comp;
+  enum { START, T_PRODUCT, V_PRODUCT, V_DONE, M_DONE, NEV };
+  cudaEvent_t ev[NEV] = {};
+  cudaError_t e = cudaSuccess;
+  for (auto& x : ev)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
+  auto record = [&](int i, cudaStream_t s) { if (e == cudaSuccess) e = cudaEventRecord(ev[i], s); };
+  auto wait = [&](cudaStream_t s, int i) { if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev[i], 0); };
+  auto synth = [&](cudaStream_t s, const double* tor, const double* pol, double2* F) {
+    SynthArgs a{};
+    a.table0 = h->d_dP;
+    a.table1 = h->d_Q;
+    a.coef[0] = pol;
+    a.coef[1] = tor;
+    a.nf = 1;
+    a.out = F;
+    launch_synth_fp64(s, d, h->d_moff, a, true);
+  };
+  auto curl = [&](cudaStream_t s, int tor, int work) {
+    launch_curl(s, d, h->d_lof, h->d_rinv, h->d_rinv2, h->d_d1, h->d_d2, h->field(tor), h->field(tor + 1),
+                h->work(work), h->work(work + 1));
+  };
+  // four components (field and curl) to their consecutive grids
+  auto grids = [&](cudaStream_t s, const double2* F, int grid) {
+    launch_fft_synth<double>(s, d, h->plan, h->d_tw, F, h->grid(grid), 4, G);
+  };
+  auto analysis = [&](cudaStream_t s, int grid, double2* F, double* tor, double* pol, int epi) {
+    launch_fft_analysis<double>(s, d, h->plan, h->d_tw, h->grid(grid), G, h->d_w, F, 2);
+    AnalysisArgs a{};
+    a.table0 = h->d_dP;
+    a.table1 = h->d_Q;
+    a.in = F;
+    a.out[0] = tor;
+    a.out[1] = pol;
+    a.nf = 1;
+    a.epi = epi;
+    launch_analysis_fp64(s, d, h->d_moff, a);
+  };
+  record(START, s0);
+  wait(s1, START);
+  wait(s2, START);
+  // temperature
+  launch_gradients(s0, d, h->d_lof, h->d_mof, h->d_rinv, h->d_d1, h->field(F_TEMP), h->work(0), h->work(1), h->work(2));
+  const double* coef[4] = {h->field(F_TEMP), h->work(0), h->work(1), h->work(2)};
+  int st = synth_scalar(h, coef, 4, h->grid(GD_GRID_T));
+  launch_temperature_advection<double>(s0, d, h->grid(GD_GRID_U_TH), h->grid(GD_GRID_U_PH), h->grid(GD_GRID_GTH),
+                                       h->grid(GD_GRID_GPH), h->grid(GD_GRID_GR), h->d_sources, h->grid(GD_GRID_TADV));
+  record(T_PRODUCT, s0);
+  double* out[1] = {h->nlf(F_TEMP)};
+  if (st == GD_OK) st = analysis_scalar(h, h->grid(GD_GRID_TADV), 1, out);
+  regular_nl(h, F_TEMP, 1);
+  scalar_bc(h, F_TEMP);
+  // velocity
+  synth(s1, h->field(F_UTOR), h->field(F_UPOL), Fv);
+  curl(s1, F_UTOR, 3);
+  synth(s1, h->work(3), h->work(4), Fv + 2 * comp);
+  wait(s1, T_PRODUCT);
+  grids(s1, Fv, GD_GRID_U_TH);
+  const double rf = h->c.magnetic_prandtl / h->c.ekman;
+  launch_velocity_nl<double>(s1, d, h->d_cth, h->d_sthc, rf, rf, h->c.magnetic, h->grid(GD_GRID_U_TH),
+                             h->grid(GD_GRID_U_PH), h->grid(GD_GRID_W_TH), h->grid(GD_GRID_W_PH),
+                             h->grid(GD_GRID_J_TH), h->grid(GD_GRID_J_PH), h->grid(GD_GRID_B_TH),
+                             h->grid(GD_GRID_B_PH), h->grid(GD_GRID_VADV_TH), h->grid(GD_GRID_VADV_PH));
+  record(V_PRODUCT, s1);
+  analysis(s1, GD_GRID_VADV_TH, Fv, h->nlf(F_UTOR), h->nlf(F_UPOL), EPI_VECTOR);
+  record(V_DONE, s1);
+  // magnetic field
+  synth(s2, h->field(F_BTOR), h->field(F_BPOL), Fm);
+  curl(s2, F_BTOR, 5);
+  synth(s2, h->work(5), h->work(6), Fm + 2 * comp);
+  wait(s2, V_PRODUCT);
+  grids(s2, Fm, GD_GRID_B_TH);
+  launch_induction<double>(s2, d, h->grid(GD_GRID_U_TH), h->grid(GD_GRID_U_PH), h->grid(GD_GRID_B_TH),
+                           h->grid(GD_GRID_B_PH), h->grid(GD_GRID_IND_TH), h->grid(GD_GRID_IND_PH));
+  analysis(s2, GD_GRID_IND_TH, Fm, h->nlf(F_BTOR), h->nlf(F_BPOL), EPI_CURL_INDUCTION);
+  if (d.ball) launch_regularity(s2, d, h->d_lof, h->nlf(F_BTOR), 2, h->spec_elems());
+  record(M_DONE, s2);
+  wait(s0, V_DONE);
+  wait(s0, M_DONE);
+  for (auto& x : ev)
+    if (x) cudaEventDestroy(x);
+  if (st != GD_OK) return st;
+  if (e != cudaSuccess) return fail(h, GD_ERR_CUDA, std::string("step fork: ") + cudaGetErrorString(e));
+  st = check_launch(h, "forked step");
+  return st ? st : implicit_launch(h, boot);
+}
+
 void drop_graphs(gd_handle* h) {
   h->graph_gen++;
   for (int p = 0; p < 2; ++p)
@@ -773,9 +909,13 @@ int ensure_graph(gd_handle* h, int boot) {
   cudaGraphExec_t& ge = h->gexec[h->nl_par][boot];
   if (ge) return GD_OK;
   cudaGraph_t g = nullptr;
+  ForkStreams* const f = h->d_F2 && can_fork(h) ? fork_streams(h->device) : nullptr;
+  std::unique_lock<std::mutex> lock;
+  if (f) lock = std::unique_lock<std::mutex>(f->mu);
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int s = step_sequence(h, boot);
+  int s = f ? step_sequence_forked(h, boot, f->s) : step_sequence(h, boot);
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
+  if (f) lock.unlock();
   if (s) { if (g) cudaGraphDestroy(g); return s; }
   if (e != cudaSuccess) return fail(h, GD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
   {
