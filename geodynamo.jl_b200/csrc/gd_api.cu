@@ -1026,6 +1026,8 @@ int gd_destroy(gd_handle* h) {
   if (h->mixed) mixed_destroy(h);
   for (void* p : h->t_snaps) cudaFree(p);
   if (h->t_final) cudaFree(h->t_final);
+  if (h->t_lam) cudaFree(h->t_lam);
+  if (h->t_grids) cudaFree(h->t_grids);
   for (void* p : h->allocs) cudaFree(p);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
@@ -1110,6 +1112,8 @@ int gd_step_kernels(gd_handle* h, int* count) {
   return GD_OK;
 }
 
+static int cnab2_adjoint(gd_handle* h, int field, int nf, int mode, const double* x, double* y);
+
 // Checkpointed forward run and the temperature pullback that recomputes the
 // velocity grids from its snapshots (the orchestration of the pieces above).
 static void free_tckpt(gd_handle* h) {
@@ -1119,6 +1123,13 @@ static void free_tckpt(gd_handle* h) {
   h->t_final = nullptr;
   h->t_nsteps = 0;
 }
+static void free_tscratch(gd_handle* h) {
+  for (double** p : {&h->t_lam, &h->t_grids}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  h->t_lam_n = h->t_grids_n = 0;
+}
 
 int gd_temperature_forward(gd_handle* h, int nsteps, int checkpoint_every) {
   if (!h || nsteps < 1 || checkpoint_every < 1) return h ? fail(h, GD_ERR_ARG, "need nsteps, checkpoint_every >= 1") : GD_ERR_ARG;
@@ -1126,20 +1137,34 @@ int gd_temperature_forward(gd_handle* h, int nsteps, int checkpoint_every) {
     return fail(h, GD_ERR_UNSUPPORTED, "the temperature pullback is of the FP64 CNAB2 step");
   if (h->d.nseg > 1 || h->d.ball) return refuse_layout(h, "the temperature pullback");
   CK(cudaSetDevice(h->device));
-  free_tckpt(h);
+  h->t_nsteps = 0;
   size_t nb = 0;
   gd_snapshot_bytes(h, &nb);
   const int nseg = (nsteps + checkpoint_every - 1) / checkpoint_every;
+  // the buffers of the run before serve again (all snapshots of a handle have
+  // one size); those beyond this run's number are given back
+  while ((int)h->t_snaps.size() > nseg) {
+    cudaFree(h->t_snaps.back());
+    h->t_snaps.pop_back();
+  }
+  auto grab = [&](void** p) {
+    if (cudaMalloc(p, nb) == cudaSuccess) return true;
+    cudaGetLastError();
+    free_tscratch(h);
+    return cudaMalloc(p, nb) == cudaSuccess;
+  };
   h->t_s0 = h->step_count;
   for (int k = 0; k < nseg; ++k) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, nb) != cudaSuccess) { free_tckpt(h); return fail(h, GD_ERR_CUDA, "out of device memory for snapshots"); }
-    h->t_snaps.push_back(p);
-    int s = gd_snapshot(h, p, 0);
+    if (k == (int)h->t_snaps.size()) {
+      void* p = nullptr;
+      if (!grab(&p)) { free_tckpt(h); return fail(h, GD_ERR_CUDA, "out of device memory for snapshots"); }
+      h->t_snaps.push_back(p);
+    }
+    int s = gd_snapshot(h, h->t_snaps[k], 0);
     if (s == GD_OK) s = gd_step(h, std::min(checkpoint_every, nsteps - k * checkpoint_every));
     if (s) { free_tckpt(h); return s; }
   }
-  if (cudaMalloc(&h->t_final, nb) != cudaSuccess) { free_tckpt(h); return fail(h, GD_ERR_CUDA, "out of device memory"); }
+  if (!h->t_final && !grab(&h->t_final)) { free_tckpt(h); return fail(h, GD_ERR_CUDA, "out of device memory"); }
   int s = gd_snapshot(h, h->t_final, 0);
   if (s) { free_tckpt(h); return s; }
   h->t_nsteps = nsteps;
@@ -1169,34 +1194,37 @@ static int temperature_pullback_impl(gd_handle* h, const double* lam_re, const d
   const int ng = vel ? 4 : 2;  // grids kept per step: u_th, u_ph (and G_th T, G_ph T)
   auto boot = [&](int n) { return ab1 || h->t_s0 + n == 0; };
   // temperature: lam, psi1, psi2, tmp, nlt; velocity: lam, psi1, psi2, tmp, nlt, src (2 se each)
-  double *lam = nullptr, *ust = nullptr;
-  if (cudaMalloc(&lam, (5 + (vel ? 12 : 0)) * se * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&ust, (size_t)C * ng * G * sizeof(double)) != cudaSuccess) {
-    if (lam) cudaFree(lam);
-    return fail(h, GD_ERR_CUDA, "out of device memory for the pullback");
+  const size_t lam_n = (5 + (vel ? 12 : 0)) * se, ust_n = (size_t)C * ng * G;
+  if (h->t_lam_n < lam_n || h->t_grids_n < ust_n) {
+    free_tscratch(h);
+    if (cudaMalloc(&h->t_lam, lam_n * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&h->t_grids, ust_n * sizeof(double)) != cudaSuccess) {
+      free_tscratch(h);
+      return fail(h, GD_ERR_CUDA, "out of device memory for the pullback");
+    }
+    h->t_lam_n = lam_n;
+    h->t_grids_n = ust_n;
   }
+  double *lam = h->t_lam, *const ust = h->t_grids;
   double *psi1 = lam + se, *psi2 = psi1 + se, *tmp = psi2 + se, *nlt = tmp + se;
   double* ul = nlt + se;  // velocity block
   double *upsi1 = ul + 2 * se, *upsi2 = upsi1 + 2 * se, *utmp = upsi2 + 2 * se, *unlt = utmp + 2 * se,
          *usrc = unlt + 2 * se;
   auto done = [&](int st) {
-    cudaFree(lam);
-    cudaFree(ust);
+    h->hold_sync = false;
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess && st == GD_OK)
+      st = fail(h, GD_ERR_CUDA, "temperature pullback");
     return st;
   };
-  auto usolve = [&](const double* x, double* y) {  // D S^-T C per potential
-    int st = gd_cnab2_adjoint(h, GD_U_TOR, 0, x, y);
-    return st ? st : gd_cnab2_adjoint(h, GD_U_POL, 0, x + se, y + se);
-  };
+  auto usolve = [&](const double* x, double* y) { return cnab2_adjoint(h, GD_U_TOR, 2, 0, x, y); };  // D S^-T C
+  h->hold_sync = true;
   int s = gd_spectral_device(h, const_cast<double*>(lam_re), const_cast<double*>(lam_im), lam, 1);
   if (s) return done(s);
   s = gd_cnab2_adjoint(h, GD_TEMP, 0, lam, psi1);
   if (s) return done(s);
-  CK(cudaMemsetAsync(psi2, 0, se * sizeof(double), h->stream));
-  if (vel) {
-    // the velocity after the run carries no cotangent of its own here
-    CK(cudaMemsetAsync(ul, 0, 12 * se * sizeof(double), h->stream));
-  }
+  cudaMemsetAsync(psi2, 0, se * sizeof(double), h->stream);
+  // the velocity after the run carries no cotangent of its own here
+  if (vel) cudaMemsetAsync(ul, 0, 12 * se * sizeof(double), h->stream);
   for (int k = nseg - 1; k >= 0 && s == GD_OK; --k) {
     const int c0 = k * C, c1 = std::min(K, c0 + C);
     s = gd_snapshot(h, h->t_snaps[k], 1);
@@ -1204,7 +1232,7 @@ static int temperature_pullback_impl(gd_handle* h, const double* lam_re, const d
       double* u = ust + (size_t)(n - c0) * ng * G;
       s = gd_grid_device(h, GD_GRID_U_TH, u);
       if (s == GD_OK) s = gd_grid_device(h, GD_GRID_U_PH, u + G);
-      if (s == GD_OK && (vel || n < c1 - 1)) s = gd_step(h, 1);
+      if (s == GD_OK && (vel || n < c1 - 1)) s = gd_step_async(h, 1);
       // the temperature gradient grids of step n's temperature phase
       if (s == GD_OK && vel) s = gd_grid_device(h, GD_GRID_GTH, u + 2 * G);
       if (s == GD_OK && vel) s = gd_grid_device(h, GD_GRID_GPH, u + 3 * G);
@@ -1221,12 +1249,11 @@ static int temperature_pullback_impl(gd_handle* h, const double* lam_re, const d
         // lambda_u^n with the source s^n of step n + 1 (usrc), then the source of step n
         launch_axpby(h->stream, 2 * se, a_n, upsi1, -b_n1, upsi2, utmp);
         s = gd_velocity_nl_adjoint(h, utmp, unlt);
-        if (s == GD_OK) s = gd_cnab2_adjoint(h, GD_U_TOR, 1, upsi1, ul);
-        if (s == GD_OK) s = gd_cnab2_adjoint(h, GD_U_POL, 1, upsi1 + se, ul + se);
+        if (s == GD_OK) s = cnab2_adjoint(h, GD_U_TOR, 2, 1, upsi1, ul);
         if (s == GD_OK) launch_axpby(h->stream, 2 * se, 1.0, ul, 1.0, unlt, ul);
         if (s == GD_OK) launch_axpby(h->stream, 2 * se, 1.0, ul, 1.0, usrc, ul);
         if (s == GD_OK && n >= 1) s = gd_temperature_u_adjoint(h, u + 2 * G, u + 3 * G, tmp, usrc);
-        if (s == GD_OK && n == 0) CK(cudaMemsetAsync(usrc, 0, 2 * se * sizeof(double), h->stream));
+        if (s == GD_OK && n == 0) cudaMemsetAsync(usrc, 0, 2 * se * sizeof(double), h->stream);
       }
       if (s == GD_OK && n > 0) {
         std::swap(psi1, psi2);
@@ -1285,7 +1312,7 @@ int gd_temperature_u_adjoint(gd_handle* h, const double* gth, const double* gph,
   launch_scale_by_order(h->stream, 4 * (size_t)d.nr, d.nlm, h->d_mof, 1.0 / tp, 2.0 / tp, out);
   s = check_launch(h, "temperature-velocity adjoint");
   if (s) return s;
-  CK(cudaStreamSynchronize(h->stream));
+  if (!h->hold_sync) CK(cudaStreamSynchronize(h->stream));
   return GD_OK;
 }
 
@@ -1450,7 +1477,7 @@ int gd_grid_device(gd_handle* h, int grid, double* dev) {
   if (h->precision != GD_PREC_FP64) return fail(h, GD_ERR_UNSUPPORTED, "device grids are the FP64 path's");
   CK(cudaSetDevice(h->device));
   CK(cudaMemcpyAsync(dev, h->grid(grid), h->grid_elems() * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  if (!h->hold_sync) CK(cudaStreamSynchronize(h->stream));
   return GD_OK;
 }
 
@@ -1482,11 +1509,12 @@ int gd_temperature_nl_adjoint(gd_handle* h, const double* u_th, const double* u_
   launch_gradients_adjoint(h->stream, h->d, h->d_lof, h->d_mof, h->d_rinv, ath, aph, out);
   s = check_launch(h, "temperature nonlinear adjoint");
   if (s) return s;
-  CK(cudaStreamSynchronize(h->stream));
+  if (!h->hold_sync) CK(cudaStreamSynchronize(h->stream));
   return GD_OK;
 }
 
-int gd_cnab2_adjoint(gd_handle* h, int field, int mode, const double* x, double* y) {
+// nf consecutive fields from `field` on, of one kind.
+static int cnab2_adjoint(gd_handle* h, int field, int nf, int mode, const double* x, double* y) {
   if (!h || !x || !y || (mode != 0 && mode != 1) || field < 0 || field >= nfields(h))
     return h ? fail(h, GD_ERR_ARG, "bad field, mode or pointer") : GD_ERR_ARG;
   if (h->scheme != GD_SCHEME_CNAB2) return fail(h, GD_ERR_UNSUPPORTED, "the adjoint is of the CNAB2 step");
@@ -1504,11 +1532,15 @@ int gd_cnab2_adjoint(gd_handle* h, int field, int mode, const double* x, double*
   }
   CK(cudaSetDevice(h->device));
   launch_cnab2_adjoint(h->stream, h->d, h->d_lof, h->d_lin, h->d_lu, types, kind, mode, h->c.dt, h->c.implicit_theta,
-                       h->c.bc_mode == 1, h->c.bc_mode == 2, x, y);
+                       h->c.bc_mode == 1, h->c.bc_mode == 2, nf, x, y);
   int s = check_launch(h, "cnab2 adjoint");
   if (s) return s;
-  CK(cudaStreamSynchronize(h->stream));
+  if (!h->hold_sync) CK(cudaStreamSynchronize(h->stream));
   return GD_OK;
+}
+
+int gd_cnab2_adjoint(gd_handle* h, int field, int mode, const double* x, double* y) {
+  return cnab2_adjoint(h, field, 1, mode, x, y);
 }
 
 int gd_derivatives(gd_handle* h, int j0, int j1) {
@@ -1820,7 +1852,7 @@ int gd_velocity_nl_adjoint(gd_handle* h, const double* psi, double* out) {
   launch_scale_by_order(h->stream, 4 * (size_t)d.nr, d.nlm, h->d_mof, 1.0 / tp, 2.0 / tp, out);
   s = check_launch(h, "velocity nonlinear adjoint");
   if (s) return s;
-  CK(cudaStreamSynchronize(h->stream));
+  if (!h->hold_sync) CK(cudaStreamSynchronize(h->stream));
   return GD_OK;
 }
 

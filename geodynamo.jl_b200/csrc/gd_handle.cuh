@@ -76,6 +76,11 @@ struct gd_handle {
   std::vector<void*> t_snaps;
   void* t_final = nullptr;
   int t_nsteps = 0, t_every = 0;
+  // pullback scratch, kept for the next call: cotangents and the recomputed grids of a segment
+  double *t_lam = nullptr, *t_grids = nullptr;
+  size_t t_lam_n = 0, t_grids_n = 0;
+  // the pieces of a pullback follow each other on the stream without waiting
+  bool hold_sync = false;
   long t_s0 = 0;
   double* d_tauc = nullptr;   // per segment: the six tau constants
   double* d_tau = nullptr;    // tau1, tau2, tau_in, tau_out on the radial nodes

@@ -240,7 +240,7 @@ void launch_scale_by_degree(cudaStream_t s, size_t nrows, int nlm, const int* lo
 // Temperature adjoint pieces (gd_adjoint.cu).
 void launch_cnab2_adjoint(cudaStream_t s, const Dims& d, const int* lof, const double* lin, const double* lu,
                           const int* types, int kind, int mode, double dt, double theta, int clamp_rows, int bc_rows,
-                          const double* x, double* y);
+                          int nf, const double* x, double* y);  // nf fields of one kind, consecutive
 void launch_gradients_adjoint(cudaStream_t s, const Dims& d, const int* lof, const int* mof, const double* rinv,
                               const double* gth, const double* gph, double* out);
 void launch_neg_product(cudaStream_t s, size_t n, const double* u, const double* g, double* out);
