@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256, 2) k_synth_scalar(Dims d, const int* __re
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (n0 + nw + 8 * j < Ntot)  // column blocks past the last column stay zero
+          if (n0 + nw + 8 * j < Ntot && th0 + thw + 16 * i < d.nth)  // blocks past the last column or row stay zero
             dmma16(acc[2 * i][j][0], acc[2 * i][j][1], acc[2 * i + 1][j][0], acc[2 * i + 1][j][1], af[i], bf[j]);
     }
   }
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(256, 2) k_synth_vector(Dims d, const int* __re
         for (int y = 0; y < 2; ++y)
 #pragma unroll
           for (int j = 0; j < 2; ++j)
-            if (n0 + nw + 8 * j < Ntot)
+            if (n0 + nw + 8 * j < Ntot && th0 + thw < d.nth)
               dmma16(acc[x][y][0][j][0], acc[x][y][0][j][1], acc[x][y][1][j][0], acc[x][y][1][j][1], af[x],
                      bf[y][j]);
     }
@@ -509,6 +509,10 @@ __global__ void __launch_bounds__(256, 2) k_analysis_scalar(Dims d, const int* _
     if (c < nch) load(c);
     cpa_commit();
   }
+  // a warp whose degrees all lie past L, or whose columns past the last, only loads
+  // (at nr = 33 the third column tile holds 2 of 32 columns, and on average a quarter
+  // of the 64-degree tiles' rows lie past L: vector analysis 258 -> 236 us at lmax 255)
+  const bool active = l0 + 2 * lw + par <= d.L && n0 + nw < Ntot;
   for (int ch = 0; ch < nch; ++ch) {
     cpa_wait<LEG_STAGES - 2>();
     __syncthreads();
@@ -516,6 +520,7 @@ __global__ void __launch_bounds__(256, 2) k_analysis_scalar(Dims d, const int* _
     cpa_commit();
     const double* As = smem + (ch % LEG_STAGES) * SA_STAGE;
     const double* Bs = As + SA_TL * SA_SA;
+    if (!active) continue;
     // two K steps of 8 colatitudes: th0 = 8 ks + t and th0 + 4
 #pragma unroll
     for (int ks = 0; ks < SA_KC / 8; ++ks) {
@@ -532,7 +537,8 @@ __global__ void __launch_bounds__(256, 2) k_analysis_scalar(Dims d, const int* _
         bf[j][1] = Bs[(par * SA_KC + th1) * SA_SB + nw + 8 * j + g];
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) dmma16(acc[0][j][0], acc[0][j][1], acc[1][j][0], acc[1][j][1], af, bf[j]);
+      for (int j = 0; j < 4; ++j)
+        if (n0 + nw + 8 * j < Ntot) dmma16(acc[0][j][0], acc[0][j][1], acc[1][j][0], acc[1][j][1], af, bf[j]);
     }
   }
   cpa_wait<0>();
@@ -633,6 +639,7 @@ __global__ void __launch_bounds__(256, 2) k_analysis_vector(Dims d, const int* _
     if (c < nch) load(c);
     cpa_commit();
   }
+  const bool active = l0 + 2 * lw + par <= d.L && n0 + nw < Ntot;  // as in the scalar analysis
   for (int ch = 0; ch < nch; ++ch) {
     cpa_wait<LEG_STAGES - 2>();
     __syncthreads();
@@ -640,6 +647,7 @@ __global__ void __launch_bounds__(256, 2) k_analysis_vector(Dims d, const int* _
     cpa_commit();
     const double* As = smem + (ch % LEG_STAGES) * VA_STAGE;
     const double* Bs = As + 2 * VA_TL * VA_SA;
+    if (!active) continue;
 #pragma unroll
     for (int ks = 0; ks < VA_KC / 8; ++ks) {
       const int th0 = 8 * ks + t, th1 = th0 + 4;
@@ -667,6 +675,7 @@ __global__ void __launch_bounds__(256, 2) k_analysis_vector(Dims d, const int* _
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
+        if (n0 + nw + 8 * j >= Ntot) continue;
         dmma16(acc[0][0][j][0], acc[0][0][j][1], acc[0][1][j][0], acc[0][1][j][1], aD, bth[0][j]);
         dmma16(acc[1][0][j][0], acc[1][0][j][1], acc[1][1][j][0], acc[1][1][j][1], aD, bph[0][j]);
         dmma16(acc[2][0][j][0], acc[2][0][j][1], acc[2][1][j][0], acc[2][1][j][1], aQ, bth[1][j]);
