@@ -287,7 +287,7 @@ int setup(gd_handle* h) {
   h->fac_stride = (h->var_op.back() / nbw + (size_t)4 * h->var_n.back() * (d.L + 1)) * 5;
   AL(h->d_fac, (c.bc_mode == 2 ? 4 : 1) * h->fac_stride);
   AL(h->d_row, h->fac_stride / 5 / (d.L + 1) * (nbw + 1));
-  AL(h->d_tw, 2 * (size_t)d.nlon); AL(h->d_twf, 2 * (size_t)d.nlon);
+  AL(h->d_tw, 4 * (size_t)d.nlon); AL(h->d_twf, 4 * (size_t)d.nlon);
   AL(h->d_state, NFIELD * h->spec_elems()); AL(h->d_nl, NFIELD * h->spec_elems());
   AL(h->d_prev, NFIELD * h->spec_elems());
   AL(h->d_work, NWORK * h->spec_elems());

@@ -4,8 +4,12 @@
 // Each CTA transforms `tb` north/south row pairs of one (component, shell):
 // the two real rows are packed into one complex sequence (north = real part,
 // south = imaginary part) and transformed with a shared-memory Stockham
-// mixed-radix FFT that ping-pongs between two buffers (radix 16 passes for
-// the power-of-two part, then 8/4/2, 3 and 5; nlon = 768 takes 16 x 16 x 3).
+// mixed-radix FFT (radix 16 passes for the power-of-two part, then 8/4/2, 3 and
+// 5; nlon = 768 takes 16 x 16 x 3): with a plan at run time between two buffers,
+// at the compile-time lengths within one (ct_run), the analysis' first pass reading
+// the grid and the synthesis' last one writing it.  Measured (FP64, lmax 255, 33
+// shells, all of a step's transforms, two buffers -> one): synthesis 537 -> 403 us,
+// analysis 313 -> 172 us.
 //
 // Synthesis consumes the Legendre output F[comp][r][m][s][ith] and writes
 // grid rows [comp][r][theta][phi].  Analysis writes the Gauss-weighted folds
@@ -122,26 +126,28 @@ __global__ void __launch_bounds__(256) k_fft_analysis(Dims d, FftPlan p, const t
 }
 
 template <typename RT, int N>
-__global__ void __launch_bounds__(256) k_fft_synth_ct(Dims d, const typename C2<RT>::T* __restrict__ tw,
-                                                      const typename C2<RT>::T* __restrict__ F, RT* __restrict__ grid,
-                                                      size_t grid_comp_stride) {
+__global__ void __launch_bounds__(CtGeom<RT, N>::NT, CtGeom<RT, N>::MINB)
+k_fft_synth_ct(Dims d, const typename C2<RT>::T* __restrict__ tw,
+               const typename C2<RT>::T* __restrict__ F, RT* __restrict__ grid,
+               size_t grid_comp_stride) {
   typedef typename C2<RT>::T C;
-  constexpr int RS = CtGeom<RT, N>::RS, TB = CtGeom<RT, N>::TB;
+  constexpr int RS = CtGeom<RT, N>::RS, TB = CtGeom<RT, N>::TB, NT = CtGeom<RT, N>::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* bufA = reinterpret_cast<C*>(smem_raw);
-  C* bufB = bufA + TB * RS;
+  C* buf = reinterpret_cast<C*>(smem_raw);
   const int M = d.M;
   const int i0 = blockIdx.x * TB;
   const int r = blockIdx.y, comp = blockIdx.z;
   const int rows = min(TB, d.nth - i0);
-  for (int e = threadIdx.x; e < TB * N; e += kThreads) {
-    const int ii = e / N, k = e - ii * N;
-    if (k > M && k < N - M) { bufA[ii * RS + pidx(k)].x = 0; bufA[ii * RS + pidx(k)].y = 0; }
+  for (int k = M + 1 + threadIdx.x; k < N - M; k += NT) {
+    C z; z.x = 0; z.y = 0;
+#pragma unroll
+    for (int ii = 0; ii < TB; ++ii) buf[ii * RS + pidx(k)] = z;
   }
   const size_t fbase = ((size_t)(comp * d.nr + r) * (M + 1)) * 2 * d.nth + i0;
-  for (int e = threadIdx.x; e < (M + 1) * TB; e += kThreads) {
+#pragma unroll 4
+  for (int e = threadIdx.x; e < (M + 1) * TB; e += NT) {
     const int m = e / TB, ii = e - m * TB;
-    C* row = bufA + ii * RS;
+    C* row = buf + ii * RS;
     C fn, fs;
     if (ii < rows) {
       fn = F[fbase + ((size_t)m * 2 + 0) * d.nth + ii];
@@ -160,51 +166,51 @@ __global__ void __launch_bounds__(256) k_fft_synth_ct(Dims d, const typename C2<
     }
   }
   __syncthreads();
-  const C* res = ct_passes<N, TB, 0, 1, C>(bufA, bufB, tw);
   RT* gbase = grid + grid_comp_stride * comp + (size_t)r * d.nlat * N;
-  for (int e = threadIdx.x; e < rows * N; e += kThreads) {
-    const int ii = e / N, j = e - ii * N;
-    const C z = res[ii * RS + pidx(j)];
+  PassThrough ld;
+  auto st = [&](int ii, int j, C z) {
+    if (ii >= rows) return;
     const int ith = i0 + ii;
     gbase[(size_t)ith * N + j] = z.x;
     gbase[(size_t)(d.nlat - 1 - ith) * N + j] = -z.y;
-  }
+  };
+  ct_run<N, TB, RS, 0, 1, C, NT, true, false>(buf, tw + N, ld, st);
 }
 
 template <typename RT, int N>
-__global__ void __launch_bounds__(256) k_fft_analysis_ct(Dims d, const typename C2<RT>::T* __restrict__ tw,
-                                                         const RT* __restrict__ grid, size_t grid_comp_stride,
-                                                         const double* __restrict__ w,
-                                                         typename C2<RT>::T* __restrict__ G) {
+__global__ void __launch_bounds__(CtGeom<RT, N>::NT, CtGeom<RT, N>::MINB)
+k_fft_analysis_ct(Dims d, const typename C2<RT>::T* __restrict__ tw,
+                  const RT* __restrict__ grid, size_t grid_comp_stride,
+                  const double* __restrict__ w,
+                  typename C2<RT>::T* __restrict__ G) {
   typedef typename C2<RT>::T C;
-  constexpr int RS = CtGeom<RT, N>::RS, TB = CtGeom<RT, N>::TB;
+  constexpr int RS = CtGeom<RT, N>::RS, TB = CtGeom<RT, N>::TB, NT = CtGeom<RT, N>::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* bufA = reinterpret_cast<C*>(smem_raw);
-  C* bufB = bufA + TB * RS;
+  C* buf = reinterpret_cast<C*>(smem_raw);
   const int M = d.M;
   const int i0 = blockIdx.x * TB;
   const int r = blockIdx.y, comp = blockIdx.z;
   const int rows = min(TB, d.nth - i0);
   const RT* gbase = grid + grid_comp_stride * comp + (size_t)r * d.nlat * N;
-  for (int e = threadIdx.x; e < TB * N; e += kThreads) {
-    const int ii = e / N, j = e - ii * N;
+  auto ld = [&](int ii, int j) {
     C z; z.x = 0; z.y = 0;
     if (ii < rows) {
       const int ith = i0 + ii;
       z.x = gbase[(size_t)ith * N + j];
       z.y = gbase[(size_t)(d.nlat - 1 - ith) * N + j];
     }
-    bufA[ii * RS + pidx(j)] = z;
-  }
-  __syncthreads();
-  const C* res = ct_passes<N, TB, 0, 1, C>(bufA, bufB, tw);
+    return z;
+  };
+  PassThrough st;
+  ct_run<N, TB, RS, 0, 1, C, NT, false, true>(buf, tw + N, ld, st);
   const RT sc = (RT)(2.0 * 3.14159265358979323846 / N);
   const size_t gb = ((size_t)(comp * d.nr + r) * (M + 1)) * 2 * d.nth;
-  for (int e = threadIdx.x; e < (M + 1) * TB; e += kThreads) {
+#pragma unroll 2
+  for (int e = threadIdx.x; e < (M + 1) * TB; e += NT) {
     const int m = e / TB, ii = e - m * TB;
     if (ii >= rows) continue;
     const int ith = i0 + ii;
-    const C* row = res + ii * RS;
+    const C* row = buf + ii * RS;
     const C zk = row[pidx(m)];
     C zn = row[pidx(m == 0 ? 0 : N - m)];
     zn.y = -zn.y;
@@ -234,28 +240,30 @@ __global__ void __launch_bounds__(256) k_fft_analysis_ct(Dims d, const typename 
 // k_fft_analysis_ct -> widen-and-add, in the same order, so the result is the
 // same to the last bit; the grids only stay in shared memory.
 template <int N>
-__global__ void __launch_bounds__(256) k_coriolis_fused(Dims d, const double2* __restrict__ tw,
-                                                        const double2* __restrict__ F, const double* __restrict__ cth,
-                                                        const double* __restrict__ sth, double rf,
-                                                        const double* __restrict__ w, const float2* __restrict__ g32,
-                                                        double2* __restrict__ G) {
+__global__ void __launch_bounds__(CtGeom<double, N>::NT, CtGeom<double, N>::MINB)
+k_coriolis_fused(Dims d, const double2* __restrict__ tw,
+                 const double2* __restrict__ F, const double* __restrict__ cth,
+                 double rf,
+                 const double* __restrict__ w, const float2* __restrict__ g32,
+                 double2* __restrict__ G) {
   typedef double2 C;
-  constexpr int RS = CtGeom<double, N>::RS, TB = CtGeom<double, N>::TB;
+  constexpr int RS = CtGeom<double, N>::RS, TB = CtGeom<double, N>::TB, NT = CtGeom<double, N>::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* bufA = reinterpret_cast<C*>(smem_raw);
-  C* bufB = bufA + TB * RS;
+  C* buf = reinterpret_cast<C*>(smem_raw);
   const int M = d.M;
   const int i0 = blockIdx.x * TB;
   const int r = blockIdx.y, oc = blockIdx.z, sc = 1 - oc;
   const int rows = min(TB, d.nth - i0);
-  for (int e = threadIdx.x; e < TB * N; e += kThreads) {
-    const int ii = e / N, k = e - ii * N;
-    if (k > M && k < N - M) { bufA[ii * RS + pidx(k)].x = 0; bufA[ii * RS + pidx(k)].y = 0; }
+  for (int k = M + 1 + threadIdx.x; k < N - M; k += NT) {
+    C z; z.x = 0; z.y = 0;
+#pragma unroll
+    for (int ii = 0; ii < TB; ++ii) buf[ii * RS + pidx(k)] = z;
   }
   const size_t fbase = ((size_t)(sc * d.nr + r) * (M + 1)) * 2 * d.nth + i0;
-  for (int e = threadIdx.x; e < (M + 1) * TB; e += kThreads) {
+#pragma unroll 2
+  for (int e = threadIdx.x; e < (M + 1) * TB; e += NT) {
     const int m = e / TB, ii = e - m * TB;
-    C* row = bufA + ii * RS;
+    C* row = buf + ii * RS;
     C fn, fs;
     if (ii < rows) {
       fn = F[fbase + ((size_t)m * 2 + 0) * d.nth + ii];
@@ -274,39 +282,37 @@ __global__ void __launch_bounds__(256) k_coriolis_fused(Dims d, const double2* _
     }
   }
   __syncthreads();
-  C* res = ct_passes<N, TB, 0, 1, C>(bufA, bufB, tw);
   // grid rows: north z.x, south -z.y; the products packed as (north, south)
   const double mrf = -(d.rfs ? d.rfs[r] : rf);
-  for (int e = threadIdx.x; e < TB * N; e += kThreads) {
-    const int ii = e / N, j = e - ii * N;
-    C* at = res + ii * RS + pidx(j);
-    C z = *at, o;
-    if (ii < rows) {
-      const int tidx = j < d.nlat - 1 ? j : d.nlat - 1;
-      const double ct = cth[tidx], st = sth[tidx];
-      const double ur = 0;
-      const double vN = z.x, vS = -z.y;
-      if (oc == 0) {
-        const double ztN = -ct * vN, ztS = -ct * vS;
-        o.x = mrf * ztN; o.y = mrf * ztS;
-      } else {
-        const double zpN = ct * vN + st * ur, zpS = ct * vS + st * ur;
-        o.x = mrf * zpN; o.y = mrf * zpS;
-      }
+  PassThrough id;
+  auto product = [&](int, int j, C z) {
+    const int tidx = j < d.nlat - 1 ? j : d.nlat - 1;
+    const double ct = cth[tidx];
+    const double st_ur = 0;  // sin(theta) u_r, u_r = 0
+    const double vN = z.x, vS = -z.y;
+    C o;
+    if (oc == 0) {
+      const double ztN = -ct * vN, ztS = -ct * vS;
+      o.x = mrf * ztN; o.y = mrf * ztS;
     } else {
-      o.x = 0; o.y = 0;
+      const double zpN = ct * vN + st_ur, zpS = ct * vS + st_ur;
+      o.x = mrf * zpN; o.y = mrf * zpS;
     }
-    *at = o;
-  }
-  __syncthreads();
-  C* out = ct_passes<N, TB, 0, 1, C>(res, res == bufA ? bufB : bufA, tw);
+    return o;
+  };
+  ct_run<N, TB, RS, 0, 1, C, NT, true, true>(buf, tw + N, id, product);
+  // the roots are read again: kept from the first transform they spill (500 bytes a thread)
+  const C* tw2 = tw + N;
+  asm volatile("" : "+l"(tw2));
+  ct_run<N, TB, RS, 0, 1, C, NT, true, true>(buf, tw2, id, id);
   const double scl = 2.0 * 3.14159265358979323846 / N;
   const size_t gb = ((size_t)(oc * d.nr + r) * (M + 1)) * 2 * d.nth;
-  for (int e = threadIdx.x; e < (M + 1) * TB; e += kThreads) {
+#pragma unroll 2
+  for (int e = threadIdx.x; e < (M + 1) * TB; e += NT) {
     const int m = e / TB, ii = e - m * TB;
     if (ii >= rows) continue;
     const int ith = i0 + ii;
-    const C* row = out + ii * RS;
+    const C* row = buf + ii * RS;
     const C zk = row[pidx(m)];
     C zn = row[pidx(m == 0 ? 0 : N - m)];
     zn.y = -zn.y;
@@ -329,26 +335,26 @@ __global__ void __launch_bounds__(256) k_coriolis_fused(Dims d, const double2* _
 
 template <int N>
 static void launch_cor(cudaStream_t s, const Dims& d, const void* tw, const void* F, const double* cth,
-                       const double* sth, double rf, const double* w, const float2* g32, void* G) {
+                       double rf, const double* w, const float2* g32, void* G) {
   constexpr int RS = CtGeom<double, N>::RS, TB = CtGeom<double, N>::TB;
-  const size_t sm = (size_t)2 * TB * RS * sizeof(double2);
+  const size_t sm = (size_t)TB * RS * sizeof(double2);
   allow_dynamic_smem(k_coriolis_fused<N>, sm);
   dim3 g(ceil_div(d.nth, TB), d.nr, 2);
-  k_coriolis_fused<N><<<g, kThreads, sm, s>>>(d, (const double2*)tw, (const double2*)F, cth, sth, rf, w, g32,
+  k_coriolis_fused<N><<<g, CtGeom<double, N>::NT, sm, s>>>(d, (const double2*)tw, (const double2*)F, cth, rf, w, g32,
                                               (double2*)G);
 }
 
 bool launch_coriolis_fused(cudaStream_t s, const Dims& d, int nlon, const void* tw, const void* F, const double* cth,
-                           const double* sth, double rf, const double* w, const float2* g32, void* G) {
+                           double rf, const double* w, const float2* g32, void* G) {
   switch (nlon) {
-    case 24: launch_cor<24>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
-    case 48: launch_cor<48>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
-    case 96: launch_cor<96>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
-    case 144: launch_cor<144>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
-    case 192: launch_cor<192>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
-    case 288: launch_cor<288>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
-    case 384: launch_cor<384>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
-    case 768: launch_cor<768>(s, d, tw, F, cth, sth, rf, w, g32, G); return true;
+    case 24: launch_cor<24>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    case 48: launch_cor<48>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    case 96: launch_cor<96>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    case 144: launch_cor<144>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    case 192: launch_cor<192>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    case 288: launch_cor<288>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    case 384: launch_cor<384>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    case 768: launch_cor<768>(s, d, tw, F, cth, rf, w, g32, G); return true;
     default: return false;
   }
 }
@@ -358,14 +364,14 @@ static bool launch_ct(cudaStream_t s, const Dims& d, const void* tw, const void*
                       int ncomp, bool synth, const double* w) {
   typedef typename C2<RT>::T C;
   constexpr int RS = CtGeom<RT, N>::RS, TB = CtGeom<RT, N>::TB;
-  const size_t sm = (size_t)2 * TB * RS * sizeof(C);
+  const size_t sm = (size_t)TB * RS * sizeof(C);
   allow_dynamic_smem(k_fft_synth_ct<RT, N>, 100 * 1024);
   allow_dynamic_smem(k_fft_analysis_ct<RT, N>, 100 * 1024);
   dim3 g(ceil_div(d.nth, TB), d.nr, ncomp);
   if (synth)
-    k_fft_synth_ct<RT, N><<<g, kThreads, sm, s>>>(d, (const C*)tw, (const C*)F, grid, stride);
+    k_fft_synth_ct<RT, N><<<g, CtGeom<RT, N>::NT, sm, s>>>(d, (const C*)tw, (const C*)F, grid, stride);
   else
-    k_fft_analysis_ct<RT, N><<<g, kThreads, sm, s>>>(d, (const C*)tw, grid, stride, w, (C*)const_cast<void*>(F));
+    k_fft_analysis_ct<RT, N><<<g, CtGeom<RT, N>::NT, sm, s>>>(d, (const C*)tw, grid, stride, w, (C*)const_cast<void*>(F));
   return true;
 }
 
@@ -405,12 +411,26 @@ FftPlan make_fft_plan(int nlon) {
   return p;
 }
 
+// W_n^k, then the passes' roots W_n^(r k n / (Ns R)) at [r - 1][k] (k < Ns), one pass
+// after the other (fewer than n in all): consecutive threads of the compile-time
+// kernels read consecutive entries.
 void make_twiddles(int n, std::vector<double>& tw) {
-  tw.resize(2 * (size_t)n);
+  tw.assign(4 * (size_t)n, 0.0);
   for (int k = 0; k < n; ++k) {
     const double a = -2.0 * 3.14159265358979323846 * k / n;
     tw[2 * k] = std::cos(a);
     tw[2 * k + 1] = std::sin(a);
+  }
+  const FftPlan p = make_fft_plan(n);
+  size_t o = n;
+  for (int s = 0, ns = 1; s < p.nstage; ns *= p.radix[s++]) {
+    if (ns == 1) continue;
+    const int step = n / (ns * p.radix[s]);
+    for (int r = 1; r < p.radix[s]; ++r)
+      for (int k = 0; k < ns; ++k, ++o) {
+        tw[2 * o] = tw[2 * (size_t)r * k * step];
+        tw[2 * o + 1] = tw[2 * (size_t)r * k * step + 1];
+      }
   }
 }
 

@@ -213,27 +213,41 @@ constexpr CPlan make_cplan(int n) {
 }
 template <int N> struct PlanOf { static constexpr CPlan p = make_cplan(N); };
 
+// Geometry of the in-place kernels (ct_run): one buffer of TB rows within 56 KB and
+// a thread for 12 points of them, so that a thread holds at most 16 points in every
+// pass (two radix-8, four radix-3 or three radix-4 butterflies), the radix-16 passes
+// keep three quarters of the threads busy and three blocks of 256 fit an SM's
+// registers.  What bounds the kernels are shared-memory wavefronts and, with few
+// warps, their latency; two buffers and 256 threads left five of eight warps idle in
+// the radix-16 passes of two 768-point rows.  Coriolis stage at nlon 768, 129 shells,
+// FP64: two buffers 682 us; one buffer, 16 points a thread 517, 12 points 481, 8
+// points 586; with the roots in the order of their use (make_twiddles) 443.
 template <typename RT, int N> struct CtGeom {
   typedef typename C2<RT>::T C;
-  static constexpr int RS = (N + (N >> 4)) | 1;  // padded row stride (elements)
-  static constexpr int TB0 = (int)((56 * 1024) / (2 * (size_t)RS * sizeof(C)));
-  static constexpr int TB = TB0 > 16 ? 16 : (TB0 < 1 ? 1 : TB0);
+  static constexpr int LEN = N + (N >> 4);  // padded row
+  static constexpr int P = 128 / sizeof(C);  // elements across the banks
+  static constexpr int TB0 = (int)((56 * 1024) / ((size_t)(LEN + P) * sizeof(C)));
+  static constexpr int TB = TB0 >= 16 ? 16 : TB0 >= 8 ? 8 : TB0 >= 4 ? 4 : TB0 >= 2 ? 2 : 1;
+  // row stride: = P / TB modulo P (1 from TB = P on), so that TB rows at P / TB
+  // consecutive indices, the order of the Fourier coefficients in memory, lie in P
+  // different banks
+  static constexpr int WANT = TB >= P ? 1 : P / TB;
+  static constexpr int RS = LEN + ((WANT - LEN) % P + P) % P;
+  static constexpr int NT = (TB * N / 12 + 31) / 32 * 32;
+  static constexpr int MINB = 768 / NT;  // blocks per SM: 24 warps at 80 registers a thread
 };
 
 // One compile-time Stockham pass.  Padded indices pidx(j + r * stride) are
 // formed as pidx(j) + r * (stride + stride / 16) when the stride is a multiple
 // of 16 (and as pidx(group base) + offset when a radix group cannot cross a
-// 16-element boundary), so the inner loops carry no index arithmetic.  The
-// twiddle table may live in global or shared memory.
-// PT: tw is this pass's own table [r - 1][k] (k < NS, consecutive k in
-// consecutive entries, so a warp's twiddle reads are conflict-free in shared
-// memory); otherwise tw is the full table W_N^i.
-template <int R, int N, int TB, int NS, typename C, int NT = kThreads, bool PT = false, bool XS = false>
+// 16-element boundary), so the inner loops carry no index arithmetic.  tw is
+// this pass's own table [r - 1][k] (k < NS, consecutive k in consecutive entries,
+// so a warp's twiddle reads are conflict-free in shared memory).
+template <int R, int N, int TB, int NS, typename C, int NT, bool XS>
 __device__ __forceinline__ void ct_pass(const C* __restrict__ src, C* __restrict__ dst, const C* __restrict__ tw) {
   constexpr int RS = XS ? N : (N + (N >> 4)) | 1;
   constexpr int NBF = N / R;
   constexpr int TOTAL = TB * NBF;
-  constexpr int TWSTEP = N / (NS * R);
   for (int b = threadIdx.x; b < TOTAL; b += NT) {
     const int row = b / NBF, j = b - row * NBF;
     const int k = j % NS;
@@ -252,7 +266,7 @@ __device__ __forceinline__ void ct_pass(const C* __restrict__ src, C* __restrict
     }
     if constexpr (NS > 1) {
 #pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], PT ? tw[(r - 1) * NS + k] : tw[r * k * TWSTEP]);
+      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw[(r - 1) * NS + k]);
     }
     Dft<R, C>::run(v);
     C* o = dst + row * RS;
@@ -276,28 +290,98 @@ __device__ __forceinline__ void ct_pass(const C* __restrict__ src, C* __restrict
   }
 }
 
-template <int N, int TB, int S, int NS, typename C, int NT = kThreads>
-__device__ __forceinline__ C* ct_passes(C* src, C* dst, const C* tw) {
+// One compile-time pass within one buffer: every thread takes its butterflies'
+// inputs into registers, and after a barrier the results go back to the buffer.
+// INS: inputs from the buffer, else ld(row, index); OUTS: st(row, index, value)
+// goes to the buffer, else st itself takes the value (a consumer that is
+// pointwise in the output index).  tw: the passes' roots (make_twiddles), this
+// pass's at OFF.
+template <int R, int N, int TB, int RS, int NS, typename C, int NT, int OFF, bool INS, bool OUTS, class L, class S>
+__device__ __forceinline__ void ct_pass_in_place(C* buf, const C* __restrict__ tw, L& ld, S& st) {
+  constexpr int NBF = N / R;
+  constexpr int TOTAL = TB * NBF;
+  constexpr int NIT = (TOTAL + NT - 1) / NT;
+  C v[NIT][R];
+#pragma unroll
+  for (int it = 0; it < NIT; ++it) {
+    const int b = threadIdx.x + it * NT;
+    if ((it + 1) * NT > TOTAL && b >= TOTAL) break;
+    const int row = b / NBF, j = b - row * NBF;
+    const C* s = buf + row * RS;
+    if constexpr (!INS) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[it][r] = ld(row, j + r * NBF);
+    } else if constexpr (NBF % 16 == 0) {
+      const C* sj = s + pidx(j);
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[it][r] = sj[r * (NBF + NBF / 16)];
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[it][r] = s[pidx(j + r * NBF)];
+    }
+    if constexpr (NS > 1) {
+      const int k = j % NS;
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[it][r] = cmul(v[it][r], tw[OFF + (r - 1) * NS + k]);
+    }
+    Dft<R, C>::run(v[it]);
+  }
+  if constexpr (INS && OUTS) __syncthreads();
+#pragma unroll
+  for (int it = 0; it < NIT; ++it) {
+    const int b = threadIdx.x + it * NT;
+    if ((it + 1) * NT > TOTAL && b >= TOTAL) break;
+    const int row = b / NBF, j = b - row * NBF;
+    const int k = j % NS;
+    const int base = (j / NS) * NS * R;
+    const int o0 = base + k;
+    C* o = buf + row * RS;
+    if constexpr (!OUTS) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) st(row, o0 + r * NS, v[it][r]);
+    } else if constexpr (NS % 16 == 0) {
+      C* oo = o + pidx(o0);
+#pragma unroll
+      for (int r = 0; r < R; ++r) oo[r * (NS + NS / 16)] = st(row, o0 + r * NS, v[it][r]);
+    } else if constexpr (16 % (NS * R) == 0) {
+      C* oo = o + o0 + (base >> 4);
+#pragma unroll
+      for (int r = 0; r < R; ++r) oo[r * NS] = st(row, o0 + r * NS, v[it][r]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) o[pidx(o0 + r * NS)] = st(row, o0 + r * NS, v[it][r]);
+    }
+  }
+  if constexpr (OUTS) __syncthreads();
+}
+
+struct PassThrough {
+  template <typename C> __device__ __forceinline__ C operator()(int, int, C v) const { return v; }
+};
+
+// All passes within one buffer: the first takes ld where INS is false, the last
+// gives to st (through the buffer where OUTS).
+template <int N, int TB, int RS, int S, int NS, typename C, int NT, bool INS, bool OUTS, class L, class ST, int OFF = 0>
+__device__ __forceinline__ void ct_run(C* buf, const C* __restrict__ tw, L& ld, ST& st) {
   constexpr CPlan P = PlanOf<N>::p;
-  if constexpr (S >= P.ns) {
-    return src;
+  constexpr int R = P.r[S];
+  if constexpr (S == P.ns - 1) {
+    ct_pass_in_place<R, N, TB, RS, NS, C, NT, OFF, INS, OUTS>(buf, tw, ld, st);
   } else {
-    constexpr int R = P.r[S];
-    ct_pass<R, N, TB, NS, C, NT>(src, dst, tw);
-    __syncthreads();
-    return ct_passes<N, TB, S + 1, NS * R, C, NT>(dst, src, tw);
+    PassThrough id;
+    ct_pass_in_place<R, N, TB, RS, NS, C, NT, OFF, INS, true>(buf, tw, ld, id);
+    ct_run<N, TB, RS, S + 1, NS * R, C, NT, true, OUTS, PassThrough, ST, (NS > 1 ? OFF + (R - 1) * NS : 0)>(buf, tw, id, st);
   }
 }
 
 // A compile-time pass that hands its outputs (row, natural index, value) to
 // f instead of storing them: the last pass of a transform whose consumer is
 // pointwise in the output index.
-template <int R, int N, int TB, int NS, typename C, int NT, bool PT, bool XS, class F>
+template <int R, int N, int TB, int NS, typename C, int NT, bool XS, class F>
 __device__ __forceinline__ void ct_pass_apply(const C* __restrict__ src, const C* __restrict__ tw, F& f) {
   constexpr int RS = XS ? N : (N + (N >> 4)) | 1;
   constexpr int NBF = N / R;
   constexpr int TOTAL = TB * NBF;
-  constexpr int TWSTEP = N / (NS * R);
   for (int b = threadIdx.x; b < TOTAL; b += NT) {
     const int row = b / NBF, j = b - row * NBF;
     const int k = j % NS;
@@ -316,7 +400,7 @@ __device__ __forceinline__ void ct_pass_apply(const C* __restrict__ src, const C
     }
     if constexpr (NS > 1) {
 #pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], PT ? tw[(r - 1) * NS + k] : tw[r * k * TWSTEP]);
+      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw[(r - 1) * NS + k]);
     }
     Dft<R, C>::run(v);
     const int o0 = (j / NS) * NS * R + k;
@@ -358,8 +442,7 @@ __device__ __forceinline__ void ct_fill_pass_twiddles(const float2* __restrict__
   }
 }
 
-// ct_passes with per-pass twiddle tables (ct_fill_pass_twiddles layout);
-// XS: rows in the unpadded xidx layout.
+// All passes between two buffers (tables: ct_fill_pass_twiddles); XS: rows in the unpadded xidx layout.
 template <int N, int TB, int S, int NS, typename C, int NT, int OFF = 0, bool XS = false>
 __device__ __forceinline__ C* ct_passes_pt(C* src, C* dst, const C* tw) {
   constexpr CPlan P = PlanOf<N>::p;
@@ -367,7 +450,7 @@ __device__ __forceinline__ C* ct_passes_pt(C* src, C* dst, const C* tw) {
     return src;
   } else {
     constexpr int R = P.r[S];
-    ct_pass<R, N, TB, NS, C, NT, true, XS>(src, dst, tw + OFF);
+    ct_pass<R, N, TB, NS, C, NT, XS>(src, dst, tw + OFF);
     __syncthreads();
     return ct_passes_pt<N, TB, S + 1, NS * R, C, NT, (NS > 1 ? OFF + (R - 1) * NS : OFF), XS>(dst, src, tw);
   }
@@ -379,9 +462,9 @@ __device__ __forceinline__ void ct_passes_pt_apply(C* src, C* dst, const C* tw, 
   constexpr CPlan P = PlanOf<N>::p;
   constexpr int R = P.r[S];
   if constexpr (S == P.ns - 1) {
-    ct_pass_apply<R, N, TB, NS, C, NT, true, XS>(src, tw + OFF, f);
+    ct_pass_apply<R, N, TB, NS, C, NT, XS>(src, tw + OFF, f);
   } else {
-    ct_pass<R, N, TB, NS, C, NT, true, XS>(src, dst, tw + OFF);
+    ct_pass<R, N, TB, NS, C, NT, XS>(src, dst, tw + OFF);
     __syncthreads();
     ct_passes_pt_apply<N, TB, S + 1, NS * R, C, NT, (NS > 1 ? OFF + (R - 1) * NS : OFF), XS>(dst, src, tw, f);
   }

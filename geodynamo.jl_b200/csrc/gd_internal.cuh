@@ -126,7 +126,7 @@ void make_twiddles(int n, std::vector<double>& tw);
 // (comps theta, phi) plus the FP32 folds g32; false (nothing launched) for an
 // nlon without a compile-time plan.
 bool launch_coriolis_fused(cudaStream_t s, const Dims& d, int nlon, const void* tw, const void* F, const double* cth,
-                           const double* sth, double rf, const double* w, const float2* g32, void* G);
+                           double rf, const double* w, const float2* g32, void* G);
 
 // ---- nonlinear terms (gd_nonlinear.cu) ----
 template <typename R>

@@ -570,7 +570,7 @@ int mixed_velocity_nl(gd_handle* h) {
   if (st & GD_STAGE_VEL_PRODUCTS) {
     const double rf = h->c.magnetic_prandtl / h->c.ekman;
     ProfScope p(h, "coriolis_fused_fp64");
-    fused = launch_coriolis_fused(h->stream, d, d.nlon, h->d_tw, U64, h->d_cth, h->d_sthc, rf, h->d_w, x->d_G, G64);
+    fused = launch_coriolis_fused(h->stream, d, d.nlon, h->d_tw, U64, h->d_cth, rf, h->d_w, x->d_G, G64);
   }
   if ((st & GD_STAGE_VEL_PRODUCTS) && !fused) {
     const double rf = h->c.magnetic_prandtl / h->c.ekman;
