@@ -131,11 +131,15 @@ __global__ void __launch_bounds__(256, 2) k_synth_scalar(Dims d, const int* __re
     if (c < nch) load(c);
     cpa_commit();
   }
+  // a warp whose colatitudes or columns all lie past the last one only loads (tested once
+  // here; a test at each MMA cost what it saved: lmax 255, nr 33, 218 -> 216 against 211 us)
+  const bool active = th0 + thw < d.nth && n0 + nw < Ntot;
   for (int ch = 0; ch < nch; ++ch) {
     cpa_wait<LEG_STAGES - 2>();
     __syncthreads();  // chunk ch landed; every warp is done with chunk ch - 1's stage
     if (ch + LEG_STAGES - 1 < nch) load(ch + LEG_STAGES - 1);
     cpa_commit();
+    if (!active) continue;
     const double* As = smem + (ch % LEG_STAGES) * SS_STAGE;
     const double* Bs = As + SS_KC * SS_SA;
     // two K steps of 8 degrees of this warp's parity: rows q0 (k = 8 ks + t) and q1 (k + 4);
@@ -162,7 +166,7 @@ __global__ void __launch_bounds__(256, 2) k_synth_scalar(Dims d, const int* __re
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (n0 + nw + 8 * j < Ntot && th0 + thw + 16 * i < d.nth)  // blocks past the last column or row stay zero
+          if (n0 + nw + 8 * j < Ntot)  // column blocks past the last column stay zero
             dmma16(acc[2 * i][j][0], acc[2 * i][j][1], acc[2 * i + 1][j][0], acc[2 * i + 1][j][1], af[i], bf[j]);
     }
   }
@@ -290,11 +294,13 @@ __global__ void __launch_bounds__(256, 2) k_synth_vector(Dims d, const int* __re
     if (c < nch) load(c);
     cpa_commit();
   }
+  const bool active = th0 + thw < d.nth && n0 + nw < Ntot;  // as in the scalar synthesis: 232 -> 226 us
   for (int ch = 0; ch < nch; ++ch) {
     cpa_wait<LEG_STAGES - 2>();
     __syncthreads();
     if (ch + LEG_STAGES - 1 < nch) load(ch + LEG_STAGES - 1);
     cpa_commit();
+    if (!active) continue;
     const double* As = smem + (ch % LEG_STAGES) * VS_STAGE;
     const double* Bs = As + 2 * VS_KC * VS_SA;
 #pragma unroll
@@ -324,7 +330,7 @@ __global__ void __launch_bounds__(256, 2) k_synth_vector(Dims d, const int* __re
         for (int y = 0; y < 2; ++y)
 #pragma unroll
           for (int j = 0; j < 2; ++j)
-            if (n0 + nw + 8 * j < Ntot && th0 + thw < d.nth)
+            if (n0 + nw + 8 * j < Ntot)
               dmma16(acc[x][y][0][j][0], acc[x][y][0][j][1], acc[x][y][1][j][0], acc[x][y][1][j][1], af[x],
                      bf[y][j]);
     }
