@@ -333,6 +333,17 @@ k_coriolis_fused(Dims d, const double2* __restrict__ tw,
   }
 }
 
+// Lengths with FP64 kernels of their own: products of 2, 3 and 5 near the grids of
+// truncations up to 341, the fused phases' lengths.  Other lengths run the plan at
+// run time, whose index divisions and two buffers cost 10 to 45 % of a step (33
+// shells, us, plan at run time -> its own kernels; FP64 / velocity chain in FP64):
+// nlon 64 90 -> 83 / 169 -> 159; 256 349 -> 252 / 326 -> 282; 512 1665 -> 1125 /
+// 876 -> 698; 900 5350 -> 3261 / 2724 -> 2120; faster at every length listed.
+#define GD_FFT_LENGTHS(X)                                                                                    \
+  X(24) X(40) X(48) X(64) X(80) X(96) X(100) X(108) X(128) X(144) X(160) X(180) X(192) X(200) X(216) X(256)  \
+  X(288) X(300) X(320) X(360) X(384) X(400) X(432) X(450) X(500) X(512) X(576) X(600) X(720) X(768) X(900)   \
+  X(1024)
+
 template <int N>
 static void launch_cor(cudaStream_t s, const Dims& d, const void* tw, const void* F, const double* cth,
                        double rf, const double* w, const float2* g32, void* G) {
@@ -347,14 +358,9 @@ static void launch_cor(cudaStream_t s, const Dims& d, const void* tw, const void
 bool launch_coriolis_fused(cudaStream_t s, const Dims& d, int nlon, const void* tw, const void* F, const double* cth,
                            double rf, const double* w, const float2* g32, void* G) {
   switch (nlon) {
-    case 24: launch_cor<24>(s, d, tw, F, cth, rf, w, g32, G); return true;
-    case 48: launch_cor<48>(s, d, tw, F, cth, rf, w, g32, G); return true;
-    case 96: launch_cor<96>(s, d, tw, F, cth, rf, w, g32, G); return true;
-    case 144: launch_cor<144>(s, d, tw, F, cth, rf, w, g32, G); return true;
-    case 192: launch_cor<192>(s, d, tw, F, cth, rf, w, g32, G); return true;
-    case 288: launch_cor<288>(s, d, tw, F, cth, rf, w, g32, G); return true;
-    case 384: launch_cor<384>(s, d, tw, F, cth, rf, w, g32, G); return true;
-    case 768: launch_cor<768>(s, d, tw, F, cth, rf, w, g32, G); return true;
+#define GD_COR(N) case N: launch_cor<N>(s, d, tw, F, cth, rf, w, g32, G); return true;
+    GD_FFT_LENGTHS(GD_COR)
+#undef GD_COR
     default: return false;
   }
 }
@@ -375,22 +381,24 @@ static bool launch_ct(cudaStream_t s, const Dims& d, const void* tw, const void*
   return true;
 }
 
-// Dispatch to a compile-time length when there is one.
+// Dispatch to a compile-time length when there is one (FP32 rows, of the mixed
+// path's transforms on host arrays alone, at the 3/2-rule lengths).
 template <typename RT>
 static bool launch_fixed(cudaStream_t s, const Dims& d, int n, const void* tw, const void* F, RT* grid,
                          size_t stride, int ncomp, bool synth, const double* w) {
-  switch (n) {
-    case 24: return launch_ct<RT, 24>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 40: return launch_ct<RT, 40>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 48: return launch_ct<RT, 48>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 96: return launch_ct<RT, 96>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 144: return launch_ct<RT, 144>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 192: return launch_ct<RT, 192>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 288: return launch_ct<RT, 288>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 384: return launch_ct<RT, 384>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    case 768: return launch_ct<RT, 768>(s, d, tw, F, grid, stride, ncomp, synth, w);
-    default: return false;
+#define GD_ROW(N) case N: return launch_ct<RT, N>(s, d, tw, F, grid, stride, ncomp, synth, w);
+  if constexpr (sizeof(RT) == 8) {
+    switch (n) {
+      GD_FFT_LENGTHS(GD_ROW)
+      default: return false;
+    }
+  } else {
+    switch (n) {
+      GD_ROW(24) GD_ROW(40) GD_ROW(48) GD_ROW(96) GD_ROW(144) GD_ROW(192) GD_ROW(288) GD_ROW(384) GD_ROW(768)
+      default: return false;
+    }
   }
+#undef GD_ROW
 }
 
 FftPlan make_fft_plan(int nlon) {

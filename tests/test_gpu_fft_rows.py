@@ -14,7 +14,8 @@ import workloads  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = (24, 40, 48, 96, 144, 192, 288, 384, 768)
+LENGTHS = (24, 40, 48, 64, 80, 96, 100, 108, 128, 144, 160, 180, 192, 200, 216, 256, 288, 300, 320, 360, 384, 400,
+           432, 450, 500, 512, 576, 600, 720, 768, 900, 1024)
 # the bound of every FP64 transform against the oracle (relative, max norm): sums of
 # at most 384 x 768 products, 2^-53 each
 TOL = 1e-12
