@@ -223,8 +223,7 @@ __global__ void __launch_bounds__(128) k_cnab2_adjoint(Dims d, const int* __rest
         double acc = cur[b].x;
 #pragma unroll
         for (int t = KL; t >= 1; --t) acc -= cur[b].u[t - 1] * w[t - 1];
-        double v = acc * cur[b].r;
-        v = fma(fma(-v, cur[b].d, acc), cur[b].r, v);  // the quotient's rounding
+        const double v = quotient(acc, cur[b].d, cur[b].r);
         yc[(size_t)i * NM] = v;
 #pragma unroll
         for (int t = KL - 1; t > 0; --t) w[t] = w[t - 1];

@@ -259,8 +259,8 @@ __global__ void __launch_bounds__(128, 3) k_cnab2(Dims d, const int* __restrict_
 // 64 bits, two divisions.  Here nine rows are unrolled per round, so a window
 // index is a constant; factors come as 16-byte loads at 32-bit offsets from
 // uniform bases; no column is tested (tables and windows are zero outside the
-// matrix); the stored reciprocal with one correction step stands for the
-// division.  The terms are read once, past the caches' retention, so that y
+// matrix); the stored reciprocal with one correction step (quotient()) stands for
+// the division.  The terms are read once, past the caches' retention, so that y
 // still lies in L2 when the downward pass reads it; two blocks of 128 threads
 // with a batch of loads in flight beat three without one where the columns fill
 // the chip unevenly.  Measured (B200, six-field or five-field step, before ->
@@ -458,9 +458,7 @@ __global__ void __launch_bounds__(128, 2) k_cnab2_step(Dims d, const int* __rest
           const In& v = cur[b];
           const double tr = v.yr - (v.u0.x * xr[0] + v.u0.y * xr[1] + v.u1.x * xr[2] + v.u1.y * xr[3]);
           const double ti = v.yi - (v.u0.x * xi[0] + v.u0.y * xi[1] + v.u1.x * xi[2] + v.u1.y * xi[3]);
-          double x_r = tr * v.dg.x, x_i = ti * v.dg.x;
-          x_r = fma(fma(-x_r, v.dg.y, tr), v.dg.x, x_r);
-          x_i = fma(fma(-x_i, v.dg.y, ti), v.dg.x, x_i);
+          const double x_r = quotient(tr, v.dg.y, v.dg.x), x_i = quotient(ti, v.dg.y, v.dg.x);
           // bc_mode 1 zeroes the boundary rows after the whole solve: the
           // substitution itself continues with the solved values
           const bool clamp = a.clamp_rows && (i == 0 || i == N - 1);

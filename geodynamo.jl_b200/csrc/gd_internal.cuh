@@ -66,6 +66,20 @@ __device__ __forceinline__ SegView seg_view(const Dims& d, int z) {
   return SegView{d.seg_info[3 * z], d.seg_info[3 * z + 1], d.var_off[2 * v], d.var_off[2 * v + 1]};
 }
 
+// a / d with r = __drcp_rn(d) at hand: the rounded product a r, then one step of
+// residual correction (P. W. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  With u = 2^-53 the
+// first quotient is off by at most 2u + u^2, the residual by u of itself, so before
+// its last rounding the result is off by less than 5 u^2: for normal d and 1 / d
+// it is a / d to within 1/2 + 2^-50 ulp while the residual does not underflow
+// (|a| >= 2^-968), and to within two ulps below.  Where the residual is not finite (infinite or NaN a,
+// an overflowing quotient, d zero or infinite) the first quotient is the division's
+// value already and is kept.
+__device__ __forceinline__ double quotient(double a, double d, double r) {
+  const double q = a * r, e = fma(q, d, -a);
+  return isfinite(e) ? fma(-e, r, q) : q;
+}
+
 // Analysis epilogue variants.
 enum { EPI_SCALAR = 0, EPI_VECTOR = 1, EPI_CURL_INDUCTION = 2 };
 
