@@ -631,7 +631,8 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
       if (rlast[s] >= 0) mbar_wait(&rfull[s], rlast[s] & 1, a.err, a.wait_limit);
   }
   if (!ok && (warp == 1 || warp == 2)) {
-    if (lane == 0) mma_commit(smem_addr(drain));
+    // (a commit covers the MMAs of the thread that executes it: the elected lane's)
+    if (elect_one()) mma_commit(smem_addr(drain));
     __syncwarp();
     mbar_wait(drain, 0, a.err, a.wait_limit);
   }
@@ -913,7 +914,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_analysis3(Dims d, const in
   if (!ok && issued >= 0) mbar_wait(&full[(threadIdx.x >> 7) & 1], issued & 1, a.err, a.wait_limit);
   if (!ok && warp == 8) {
     // the MMAs issued before the failure finish before tensor memory is freed
-    if (lane == 0) mma_commit(smem_addr(drain));
+    // (a commit covers the MMAs of the thread that executes it: the elected lane's)
+    if (elect_one()) mma_commit(smem_addr(drain));
     __syncwarp();
     mbar_wait(drain, 0, a.err, a.wait_limit);
   }
