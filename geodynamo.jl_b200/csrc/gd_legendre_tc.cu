@@ -97,11 +97,6 @@ __device__ __forceinline__ void issue_products(uint32_t tmem, const float* X0, c
   }
 }
 
-// mbar_wait with one outcome for the whole warp.
-__device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int* err, long long limit) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, limit));
-}
-
 // 8-deep slices with valid degrees in K chunk kc of parity p
 __device__ __forceinline__ int synth_slices(int L, int m, int p, int kc) {
   return min(TC_K / 8, (kpar(L, m, p) - TC_K * kc + 7) / 8);
@@ -383,9 +378,9 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
         const bool omit = a.omit_plus1 == G + 1 && blockIdx.x == 0;
         const int rs = G % SY_R, ru = G / SY_R;
         // the chunk's slots: vector one of the shared ones, scalar a hi / lo pair of the ring
-        if (ru >= 1 && !(VEC ? wait_all(&hempty[rs], (ru - 1) & 1, a.err, a.wait_limit)
-                             : wait_all(&sempty[2 * rs], (ru - 1) & 1, a.err, a.wait_limit) &&
-                                   wait_all(&sempty[2 * rs + 1], (ru - 1) & 1, a.err, a.wait_limit))) {
+        if (ru >= 1 && !(VEC ? mbar_wait_warp(&hempty[rs], (ru - 1) & 1, a.err, a.wait_limit)
+                             : mbar_wait_warp(&sempty[2 * rs], (ru - 1) & 1, a.err, a.wait_limit) &&
+                                   mbar_wait_warp(&sempty[2 * rs + 1], (ru - 1) & 1, a.err, a.wait_limit))) {
           ok = false;
           break;
         }
@@ -401,7 +396,7 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
         for (int x = 0; x < (VEC ? 2 : 1); ++x) {
           const int Q = VEC ? 2 * G + x : G, NS = VEC ? SY_S : SY_H, qs = Q % NS, qu = Q / NS;
           uint64_t* const fullb = VEC ? &sfull[qs] : &hfull[qs];
-          if (qu >= 1 && !wait_all(VEC ? &sempty[qs] : &hempty[qs], (qu - 1) & 1, a.err, a.wait_limit)) {
+          if (qu >= 1 && !mbar_wait_warp(VEC ? &sempty[qs] : &hempty[qs], (qu - 1) & 1, a.err, a.wait_limit)) {
             ok = false;
             break;
           }
@@ -430,7 +425,7 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
       const int n4 = ((nvalid + 7) & ~7) * (TC_K / 4);
       for (int it = 0; it < T && ok; ++it) {
         const int G = gs + it, rs = G % SY_R;
-        if (!wait_all(&rfull[rs], (G / SY_R) & 1, a.err, a.wait_limit)) {
+        if (!mbar_wait_warp(&rfull[rs], (G / SY_R) & 1, a.err, a.wait_limit)) {
           ok = false;
           break;
         }
@@ -470,7 +465,7 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
       const int nvalid = VEC ? 4 * min(32, d.nr - ct * 32) : min(NCS, Ntot - ct * NCS);
       const uint32_t ids = idesc_tf32(TC_M, (nvalid + 15) & ~15);
       const int nc = p == 0 ? nc0 : nc1;
-      if (q >= 1 && !wait_all(tempty, (q - 1) & 1, a.err, a.wait_limit)) {
+      if (q >= 1 && !mbar_wait_warp(tempty, (q - 1) & 1, a.err, a.wait_limit)) {
         ok = false;
         break;
       }
@@ -478,14 +473,14 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
         const int G = gs + synth_step_of(p, kc, nc1), hs = G % SY_H;
         const int nks = synth_slices(L, m, p, kc);
         const float* H = hst + hs * SY_SLOT;
-        if (!wait_all(&hfull[hs], (G / SY_H) & 1, a.err, a.wait_limit)) {
+        if (!mbar_wait_warp(&hfull[hs], (G / SY_H) & 1, a.err, a.wait_limit)) {
           ok = false;
           break;
         }
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           const int Q = 2 * G + x, qs = Q % SY_S;
-          if (!wait_all(&sfull[qs], (Q / SY_S) & 1, a.err, a.wait_limit)) {
+          if (!mbar_wait_warp(&sfull[qs], (Q / SY_S) & 1, a.err, a.wait_limit)) {
             ok = false;
             break;
           }
@@ -520,7 +515,7 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
     for (int tt = blockIdx.x; tt < ntiles && ok; tt += gridDim.x, ++q) {
       const int m = tt / (ntt * ncol), tile = (tt / ncol) % ntt, ct = tt % ncol;
       const int nc1 = nck_h(L, m, 1);
-      if (!mbar_wait(tfull, q & 1, a.err, a.wait_limit)) {
+      if (!mbar_wait_warp(tfull, q & 1, a.err, a.wait_limit)) {
         ok = false;
         break;
       }
@@ -818,12 +813,11 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_analysis3(Dims d, const in
   } else {
     for (int it = 0; it < T; ++it) {
       const int s = (gs + it) & 1;
-      if (!mbar_wait(&full[s], ((gs + it) >> 1) & 1, a.err, a.wait_limit)) {
+      if (!mbar_wait_warp(&full[s], ((gs + it) >> 1) & 1, a.err, a.wait_limit)) {
         ok = false;
         break;
       }
       fence_after_sync();
-      __syncwarp();
       if (elect_one()) {
         const int cc = it / ns, p = it % ns;
         const int nks = min(TC_K / 8, (d.nth - TC_K * cc + 7) / 8);

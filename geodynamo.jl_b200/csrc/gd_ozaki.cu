@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_synth_vector(Dims d, const
         const int nk = oz_nks(L, t.m, p);
         for (int ks = 0; ks < nk; ++ks) {
           const int Gs = gs++, s = Gs % S, u = Gs / S;
-          if (u >= 1 && !mbar_wait(&empty[s], (u - 1) & 1, a.err, a.wait_limit)) {
+          if (u >= 1 && !mbar_wait_warp(&empty[s], (u - 1) & 1, a.err, a.wait_limit)) {
             ok = false;
             break;
           }
@@ -377,14 +377,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_synth_vector(Dims d, const
     for (int tt = blockIdx.x; tt < ntiles && ok; tt += gridDim.x, ++q) {
       const OzTile t = oz_tile(tt, ntt, ncb);
       for (int p = 0; p < 2 && ok; ++p) {
-        if (q >= 1 && !mbar_wait(&tempty[p], (q - 1) & 1, a.err, a.wait_limit)) {
+        if (q >= 1 && !mbar_wait_warp(&tempty[p], (q - 1) & 1, a.err, a.wait_limit)) {
           ok = false;
           break;
         }
         const int nk = oz_nks(L, t.m, p);
         for (int ks = 0; ks < nk; ++ks) {
           const int Gs = gs++, s = Gs % S;
-          if (!mbar_wait(&full[s], (Gs / S) & 1, a.err, a.wait_limit)) {
+          if (!mbar_wait_warp(&full[s], (Gs / S) & 1, a.err, a.wait_limit)) {
             ok = false;
             break;
           }
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_synth_vector(Dims d, const
       bool good = true;
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        const bool w = mbar_wait(&tfull[p], q & 1, a.err, a.wait_limit);
+        const bool w = mbar_wait_warp(&tfull[p], q & 1, a.err, a.wait_limit);
         good = good && w;
         fence_after_sync();
         const bool any = w && oz_kpar(L, t.m, p) > 0;

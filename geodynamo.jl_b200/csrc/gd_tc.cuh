@@ -154,6 +154,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   }
 }
 
+// The same with one outcome for the whole warp, for warps that go on to warp-wide
+// instructions (elect.sync, tcgen05.ld, __syncwarp): near the bound some lanes
+// could see the phase complete and others give up.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err, long long limit = 0) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, limit));
+}
+
 // Round-to-nearest TF32 value of x (low 13 bits of the FP32 pattern zero).
 __device__ __forceinline__ float tf32_rn(float x) {
   uint32_t r;

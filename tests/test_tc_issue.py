@@ -55,6 +55,16 @@ def test_commits_come_from_the_lane_that_issues(name):
     assert set(commits) == issued, guards
 
 
+@pytest.mark.parametrize("name", FILES)
+def test_waits_ahead_of_warp_wide_instructions_have_one_outcome(name):
+    """Per-lane outcomes only where no warp-wide instruction follows: the loaders of
+    the analysis, and the drain of its stages, which a block-wide vote follows."""
+    per_lane = {"&empty[g]", "&empty[(gs + T - q) & 1]"}
+    used = re.findall(r"(?:[!=] ?|&& |\? |: )mbar_wait\(([^,]+),", _code(name))
+    assert set(used) <= per_lane, used
+    assert len(re.findall(r"mbar_wait_warp\(", _code(name))) >= 4
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("omit", [0, 3])
 def test_failed_vector_synthesis_drains_and_recovers(gdb, omit):
