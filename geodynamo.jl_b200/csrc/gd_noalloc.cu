@@ -7,42 +7,18 @@
 // pool holds the free memory), or a solver loop in a framework that forbids
 // allocation between its own set-up and tear-down.  This entry point serves
 // them: inputs and outputs are the caller's device buffers, and the Fourier
-// intermediate lives in a fixed-size array in the library's device image
-// instead of a cudaMalloc'd buffer.
+// intermediate is the one the handle allocated when it was created, so calls on
+// handles of their own, each on its own stream, have nothing in common.
 #include <cuda_runtime.h>
 
-#include <mutex>
 #include <string>
 
 #include "gd_handle.cuh"
 #include "gd_internal.cuh"
 
-// Scratch for the Fourier coefficients of one call: min(nfield, 4) x nr x
-// (mmax+1) x nlat complex doubles.  Every GPU that loads the library holds
-// these 64 MiB until the process exits.
+// Most Fourier coefficients a call takes: min(nfield, 4) x nr x (mmax+1) x nlat
+// complex doubles (the documented limit of the call).
 static const size_t kScratchBytes = size_t(64) << 20;
-static __device__ __align__(256) unsigned char g_fourier_scratch[size_t(64) << 20];
-
-// Device address of g_fourier_scratch, looked up once per device with that
-// device current (host code cannot use the symbol's name as a device
-// address).  The cached address belongs to the device's primary context, which
-// lives as long as the process unless the caller resets the device; the mutex
-// makes the first lookup safe when several host threads call at once.
-static std::mutex g_scratch_mu;
-static void* g_scratch_addr[64] = {};
-
-static cudaError_t scratch_address(int device, void** out) {
-  std::lock_guard<std::mutex> lock(g_scratch_mu);
-  if (!g_scratch_addr[device]) {
-    void* p = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&p, g_fourier_scratch);
-    if (e != cudaSuccess) return e;
-    if (!p) return cudaErrorInvalidSymbol;
-    g_scratch_addr[device] = p;
-  }
-  *out = g_scratch_addr[device];
-  return cudaSuccess;
-}
 
 // Makes the handle's device current for the call and restores the caller's
 // current device afterwards.
@@ -71,15 +47,10 @@ extern "C" int gd_spectral_to_physical_noalloc(gd_handle* h, int nfield, const d
                          "gd_spectral_to_physical_noalloc needs " + std::to_string(per_field * group) +
                              " bytes of Fourier scratch (min(nfield,4) x nr x (mmax+1) x nlat x 16); the fixed "
                              "maximum is " + std::to_string(kScratchBytes) + " bytes");
-  if (h->device < 0 || h->device >= 64) return gd::set_error(h, GD_ERR_ARG, "device index out of range");
   DeviceScope scope;
   cudaError_t e = scope.enter(h->device);
   if (e != cudaSuccess) return gd::set_error(h, GD_ERR_CUDA, std::string("cudaSetDevice: ") + cudaGetErrorString(e));
-  void* scratch = nullptr;
-  e = scratch_address(h->device, &scratch);
-  if (e != cudaSuccess)
-    return gd::set_error(h, GD_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-  double2* F = static_cast<double2*>(scratch);
+  double2* const F = h->d_F;  // four components
   const size_t plane = (size_t)2 * d.nr * d.nlm;  // one field: Re and Im planes
   const size_t G = (size_t)d.nlat * d.nlon * d.nr;
   for (int f0 = 0; f0 < nfield; f0 += 4) {

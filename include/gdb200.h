@@ -252,16 +252,14 @@ int gd_enforce_regularity(gd_handle* h, int field);
  * set-up.  d_coef and d_grid are the caller's device buffers in the native
  * layout: d_coef holds nfield fields of two planes (Re, Im) of nr x nlm doubles
  * with the m-major mode index j = moff[m] + (l - m); d_grid receives nfield
- * grids of nr x nlat x nlon doubles, phi fastest.  The Fourier intermediate
- * uses a fixed 64 MiB array in the library's device image instead of
- * cudaMalloc: min(nfield, 4) x nr x (mmax+1) x nlat x 16 bytes must fit, else
- * GD_ERR_CONFIG.  The first call on a device looks up that array's device
- * address; make it before any stream capture.  The cached address assumes the
- * device's primary context lives as long as the process (no device reset in
- * between).  The caller's current device is restored on return.  The array is shared by every
- * call and keeps the last call's contents (each call overwrites what it
- * reads), so calls that overlap on the GPU (other streams, other threads)
- * race.  Runs asynchronously on the handle's stream; gd_synchronize() waits. */
+ * grids of nr x nlat x nlon doubles, phi fastest.  The Fourier intermediate is
+ * the handle's own buffer, allocated with the handle; a call takes at most 64 MiB
+ * of it: min(nfield, 4) x nr x (mmax+1) x nlat x 16 bytes must fit, else
+ * GD_ERR_CONFIG.  The caller's current device is restored on return.  Runs
+ * asynchronously on the handle's stream; gd_synchronize() waits.  Calls on
+ * different handles share nothing and may overlap; a caller that captures the call
+ * and replays it on another stream orders the replay with the handle's other
+ * work. */
 int gd_spectral_to_physical_noalloc(gd_handle* h, int nfield, const double* d_coef, double* d_grid);
 
 /* ---- the reference's nonlinear and time-step functions on host arrays ---------
