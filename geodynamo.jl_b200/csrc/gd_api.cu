@@ -5,7 +5,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -778,39 +777,33 @@ bool can_fork(const gd_handle* h) {
   return h->precision == GD_PREC_FP64 && !h->ext_derivs && h->c.magnetic && !h->c.composition && 4 * comp <= FORK_BYTES;
 }
 
-// Two streams per device that carry the branches while a step is captured (the
-// graph keeps none of them): made once, held by one capture at a time.
-struct ForkStreams {
-  std::mutex mu;
-  cudaStream_t s[2] = {nullptr, nullptr};
+// The branches of a graph under capture on one stream: what the next launch
+// depends on is read and set, so they need neither streams nor events.
+struct CaptureBranches {
+  typedef std::vector<cudaGraphNode_t> Heads;
+  cudaStream_t s;
+  cudaError_t e = cudaSuccess;
+  Heads at() {
+    cudaStreamCaptureStatus st;
+    const cudaGraphNode_t* p = nullptr;
+    size_t n = 0;
+    if (e == cudaSuccess) e = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, nullptr, &p, &n);
+    return e == cudaSuccess ? Heads(p, p + n) : Heads();
+  }
+  void depend(Heads h, unsigned flags) {
+    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(s, h.data(), h.size(), flags);
+  }
+  void from(const Heads& h) { depend(h, cudaStreamSetCaptureDependencies); }
+  void join(const Heads& h) { depend(h, cudaStreamAddCaptureDependencies); }
 };
-ForkStreams* fork_streams(int device) {
-  static ForkStreams pool[64];
-  if (device < 0 || device >= 64) return nullptr;
-  ForkStreams* f = &pool[device];
-  std::lock_guard<std::mutex> lock(f->mu);
-  for (auto& s : f->s)
-    if (!s && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
-      s = nullptr;
-      cudaGetLastError();
-      return nullptr;
-    }
-  return f;
-}
 
-int step_sequence_forked(gd_handle* h, int boot, const cudaStream_t* fork) {
+int step_sequence_forked(gd_handle* h, int boot) {
   const Dims& d = h->d;
-  const cudaStream_t s0 = h->stream, s1 = fork[0], s2 = fork[1];
+  const cudaStream_t s = h->stream;
   const size_t comp = (size_t)d.nr * (d.M + 1) * d.nlat, G = h->grid_elems();
   double2 *const Fv = h->d_F2, *const Fm = h->d_F2 + 4 * comp;
-  enum { START, T_PRODUCT, V_PRODUCT, V_DONE, M_DONE, NEV };
-  cudaEvent_t ev[NEV] = {};
-  cudaError_t e = cudaSuccess;
-  for (auto& x : ev)
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
-  auto record = [&](int i, cudaStream_t s) { if (e == cudaSuccess) e = cudaEventRecord(ev[i], s); };
-  auto wait = [&](cudaStream_t s, int i) { if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev[i], 0); };
-  auto synth = [&](cudaStream_t s, const double* tor, const double* pol, double2* F) {
+  CaptureBranches br{s};
+  auto synth = [&](const double* tor, const double* pol, double2* F) {
     SynthArgs a{};
     a.table0 = h->d_dP;
     a.table1 = h->d_Q;
@@ -820,15 +813,15 @@ int step_sequence_forked(gd_handle* h, int boot, const cudaStream_t* fork) {
     a.out = F;
     launch_synth_fp64(s, d, h->d_moff, a, true);
   };
-  auto curl = [&](cudaStream_t s, int tor, int work) {
+  auto curl = [&](int tor, int work) {
     launch_curl(s, d, h->d_lof, h->d_rinv, h->d_rinv2, h->d_d1, h->d_d2, h->field(tor), h->field(tor + 1),
                 h->work(work), h->work(work + 1));
   };
   // four components (field and curl) to their consecutive grids
-  auto grids = [&](cudaStream_t s, const double2* F, int grid) {
+  auto grids = [&](const double2* F, int grid) {
     launch_fft_synth<double>(s, d, h->plan, h->d_tw, F, h->grid(grid), 4, G);
   };
-  auto analysis = [&](cudaStream_t s, int grid, double2* F, double* tor, double* pol, int epi) {
+  auto analysis = [&](int grid, double2* F, double* tor, double* pol, int epi) {
     launch_fft_analysis<double>(s, d, h->plan, h->d_tw, h->grid(grid), G, h->d_w, F, 2);
     AnalysisArgs a{};
     a.table0 = h->d_dP;
@@ -840,51 +833,49 @@ int step_sequence_forked(gd_handle* h, int boot, const cudaStream_t* fork) {
     a.epi = epi;
     launch_analysis_fp64(s, d, h->d_moff, a);
   };
-  record(START, s0);
-  wait(s1, START);
-  wait(s2, START);
+  const auto start = br.at();
   // temperature
-  launch_gradients(s0, d, h->d_lof, h->d_mof, h->d_rinv, h->d_d1, h->field(F_TEMP), h->work(0), h->work(1), h->work(2));
+  launch_gradients(s, d, h->d_lof, h->d_mof, h->d_rinv, h->d_d1, h->field(F_TEMP), h->work(0), h->work(1), h->work(2));
   const double* coef[4] = {h->field(F_TEMP), h->work(0), h->work(1), h->work(2)};
   int st = synth_scalar(h, coef, 4, h->grid(GD_GRID_T));
-  launch_temperature_advection<double>(s0, d, h->grid(GD_GRID_U_TH), h->grid(GD_GRID_U_PH), h->grid(GD_GRID_GTH),
+  launch_temperature_advection<double>(s, d, h->grid(GD_GRID_U_TH), h->grid(GD_GRID_U_PH), h->grid(GD_GRID_GTH),
                                        h->grid(GD_GRID_GPH), h->grid(GD_GRID_GR), h->d_sources, h->grid(GD_GRID_TADV));
-  record(T_PRODUCT, s0);
+  const auto t_product = br.at();
   double* out[1] = {h->nlf(F_TEMP)};
   if (st == GD_OK) st = analysis_scalar(h, h->grid(GD_GRID_TADV), 1, out);
   regular_nl(h, F_TEMP, 1);
   scalar_bc(h, F_TEMP);
+  const auto t_done = br.at();
   // velocity
-  synth(s1, h->field(F_UTOR), h->field(F_UPOL), Fv);
-  curl(s1, F_UTOR, 3);
-  synth(s1, h->work(3), h->work(4), Fv + 2 * comp);
-  wait(s1, T_PRODUCT);
-  grids(s1, Fv, GD_GRID_U_TH);
+  br.from(start);
+  synth(h->field(F_UTOR), h->field(F_UPOL), Fv);
+  curl(F_UTOR, 3);
+  synth(h->work(3), h->work(4), Fv + 2 * comp);
+  br.join(t_product);
+  grids(Fv, GD_GRID_U_TH);
   const double rf = h->c.magnetic_prandtl / h->c.ekman;
-  launch_velocity_nl<double>(s1, d, h->d_cth, h->d_sthc, rf, rf, h->c.magnetic, h->grid(GD_GRID_U_TH),
+  launch_velocity_nl<double>(s, d, h->d_cth, h->d_sthc, rf, rf, h->c.magnetic, h->grid(GD_GRID_U_TH),
                              h->grid(GD_GRID_U_PH), h->grid(GD_GRID_W_TH), h->grid(GD_GRID_W_PH),
                              h->grid(GD_GRID_J_TH), h->grid(GD_GRID_J_PH), h->grid(GD_GRID_B_TH),
                              h->grid(GD_GRID_B_PH), h->grid(GD_GRID_VADV_TH), h->grid(GD_GRID_VADV_PH));
-  record(V_PRODUCT, s1);
-  analysis(s1, GD_GRID_VADV_TH, Fv, h->nlf(F_UTOR), h->nlf(F_UPOL), EPI_VECTOR);
-  record(V_DONE, s1);
+  const auto v_product = br.at();
+  analysis(GD_GRID_VADV_TH, Fv, h->nlf(F_UTOR), h->nlf(F_UPOL), EPI_VECTOR);
+  const auto v_done = br.at();
   // magnetic field
-  synth(s2, h->field(F_BTOR), h->field(F_BPOL), Fm);
-  curl(s2, F_BTOR, 5);
-  synth(s2, h->work(5), h->work(6), Fm + 2 * comp);
-  wait(s2, V_PRODUCT);
-  grids(s2, Fm, GD_GRID_B_TH);
-  launch_induction<double>(s2, d, h->grid(GD_GRID_U_TH), h->grid(GD_GRID_U_PH), h->grid(GD_GRID_B_TH),
+  br.from(start);
+  synth(h->field(F_BTOR), h->field(F_BPOL), Fm);
+  curl(F_BTOR, 5);
+  synth(h->work(5), h->work(6), Fm + 2 * comp);
+  br.join(v_product);
+  grids(Fm, GD_GRID_B_TH);
+  launch_induction<double>(s, d, h->grid(GD_GRID_U_TH), h->grid(GD_GRID_U_PH), h->grid(GD_GRID_B_TH),
                            h->grid(GD_GRID_B_PH), h->grid(GD_GRID_IND_TH), h->grid(GD_GRID_IND_PH));
-  analysis(s2, GD_GRID_IND_TH, Fm, h->nlf(F_BTOR), h->nlf(F_BPOL), EPI_CURL_INDUCTION);
-  if (d.ball) launch_regularity(s2, d, h->d_lof, h->nlf(F_BTOR), 2, h->spec_elems());
-  record(M_DONE, s2);
-  wait(s0, V_DONE);
-  wait(s0, M_DONE);
-  for (auto& x : ev)
-    if (x) cudaEventDestroy(x);
+  analysis(GD_GRID_IND_TH, Fm, h->nlf(F_BTOR), h->nlf(F_BPOL), EPI_CURL_INDUCTION);
+  if (d.ball) launch_regularity(s, d, h->d_lof, h->nlf(F_BTOR), 2, h->spec_elems());
+  br.join(t_done);
+  br.join(v_done);
   if (st != GD_OK) return st;
-  if (e != cudaSuccess) return fail(h, GD_ERR_CUDA, std::string("step fork: ") + cudaGetErrorString(e));
+  if (br.e != cudaSuccess) return fail(h, GD_ERR_CUDA, std::string("step fork: ") + cudaGetErrorString(br.e));
   st = check_launch(h, "forked step");
   return st ? st : implicit_launch(h, boot);
 }
@@ -909,13 +900,9 @@ int ensure_graph(gd_handle* h, int boot) {
   cudaGraphExec_t& ge = h->gexec[h->nl_par][boot];
   if (ge) return GD_OK;
   cudaGraph_t g = nullptr;
-  ForkStreams* const f = h->d_F2 && can_fork(h) ? fork_streams(h->device) : nullptr;
-  std::unique_lock<std::mutex> lock;
-  if (f) lock = std::unique_lock<std::mutex>(f->mu);
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int s = f ? step_sequence_forked(h, boot, f->s) : step_sequence(h, boot);
+  int s = h->d_F2 && can_fork(h) ? step_sequence_forked(h, boot) : step_sequence(h, boot);
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-  if (f) lock.unlock();
   if (s) { if (g) cudaGraphDestroy(g); return s; }
   if (e != cudaSuccess) return fail(h, GD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
   {
