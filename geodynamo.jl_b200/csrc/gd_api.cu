@@ -23,6 +23,11 @@ namespace {
 // Largest four-component Fourier buffer of a model whose captured step runs its
 // phases side by side (step_sequence_forked); above, the kernels fill the chip.
 constexpr size_t FORK_BYTES = (size_t)64 << 20;
+// Steps with the same settings after which they do.  Capturing and destroying the
+// two graphs with branches costs 1.3 ms beyond the chain's, the saving of 15 to 30
+// steps (ensure_graph); a run that changes dt more often than this stays on the
+// chain, and one that changes it just after loses at most a fifth of its time.
+constexpr long FORK_AFTER = 64;
 
 int nfields(const gd_handle* h) { return h->c.composition ? NFIELD : NFIELD - 1; }
 
@@ -882,9 +887,12 @@ int step_sequence_forked(gd_handle* h, int boot) {
 
 void drop_graphs(gd_handle* h) {
   h->graph_gen++;
-  for (int p = 0; p < 2; ++p)
+  h->gen_steps = 0;
+  for (int p = 0; p < 2; ++p) {
     for (int i = 0; i < 2; ++i)
       if (h->gexec[p][i]) { cudaGraphExecDestroy(h->gexec[p][i]); h->gexec[p][i] = nullptr; }
+    if (h->gfork[p]) { cudaGraphExecDestroy(h->gfork[p]); h->gfork[p] = nullptr; }
+  }
 }
 
 // After a step's implicit solve: its nonlinear terms become the history of
@@ -895,13 +903,10 @@ void end_step(gd_handle* h) {
   h->step_count++;
 }
 
-// The step graph for the current nonlinear bank and bootstrap flag.
-int ensure_graph(gd_handle* h, int boot) {
-  cudaGraphExec_t& ge = h->gexec[h->nl_par][boot];
-  if (ge) return GD_OK;
+int capture_step(gd_handle* h, int boot, bool forked, cudaGraphExec_t* ge, int* kernels) {
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int s = h->d_F2 && can_fork(h) ? step_sequence_forked(h, boot) : step_sequence(h, boot);
+  int s = forked ? step_sequence_forked(h, boot) : step_sequence(h, boot);
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (s) { if (g) cudaGraphDestroy(g); return s; }
   if (e != cudaSuccess) return fail(h, GD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -917,11 +922,31 @@ int ensure_graph(gd_handle* h, int boot) {
           if (cudaGraphNodeGetType(nodes[i], &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) ++k;
         }
     }
-    h->graph_kernels[h->nl_par][boot] = k;
+    *kernels = k;
   }
-  e = cudaGraphInstantiate(&ge, g, 0);
+  e = cudaGraphInstantiate(ge, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return fail(h, GD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+  return GD_OK;
+}
+
+// The step graph for the current nonlinear bank and bootstrap flag: the chain, and
+// for small FP64 models the side-by-side form once FORK_AFTER steps have run with
+// the same settings.  Measured (B200, lmax 31, nr 32): capture and instantiation
+// 210 us (chain) and 350 us (branches) a graph; dropping the graphs when dt changes
+// 590 and 1250 us; a step 142 and 90 us.
+int ensure_graph(gd_handle* h, int boot, cudaGraphExec_t* ge, int* kernels = nullptr) {
+  const int p = h->nl_par;
+  // (a bootstrap step between others, as after restoring a start, takes the chain)
+  const bool forked = h->gen_steps >= FORK_AFTER && boot == h->c.ab_mode && h->d_F2 && can_fork(h);
+  cudaGraphExec_t& held = forked ? h->gfork[p] : h->gexec[p][boot];
+  int& count = forked ? h->fork_kernels[p] : h->graph_kernels[p][boot];
+  if (!held) {
+    const int s = capture_step(h, boot, forked, &held, &count);
+    if (s) return s;
+  }
+  *ge = held;
+  if (kernels) *kernels = count;
   return GD_OK;
 }
 
@@ -1093,10 +1118,8 @@ int gd_step_kernels(gd_handle* h, int* count) {
   if (!h || !count) return GD_ERR_ARG;
   const int boot = (h->c.ab_mode == 1 || h->step_count == 0) ? 1 : 0;
   CK(cudaSetDevice(h->device));
-  int s = ensure_graph(h, boot);
-  if (s) return s;
-  *count = h->graph_kernels[h->nl_par][boot];
-  return GD_OK;
+  cudaGraphExec_t ge = nullptr;
+  return ensure_graph(h, boot, &ge, count);
 }
 
 static int cnab2_adjoint(gd_handle* h, int field, int nf, int mode, const double* x, double* y);
@@ -2246,9 +2269,11 @@ int gd_step_async(gd_handle* h, int nsteps) {
       int s = step_sequence(h, boot);
       if (s) return s;
     } else {
-      int s = ensure_graph(h, boot);
+      cudaGraphExec_t ge = nullptr;
+      int s = ensure_graph(h, boot, &ge);
       if (s) return s;
-      CK(cudaGraphLaunch(h->gexec[h->nl_par][boot], h->stream));
+      CK(cudaGraphLaunch(ge, h->stream));
+      h->gen_steps++;
     }
     end_step(h);
   }

@@ -103,6 +103,10 @@ struct gd_handle {
   cudaGraphExec_t gexec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [nl_par][boot]
   int graph_gen = 0;  // bumped whenever captured step graphs become stale
   int graph_kernels[2][2] = {{0, 0}, {0, 0}};  // kernel nodes of each captured step graph
+  // side-by-side graphs [nl_par], which take over after some steps of a generation (ensure_graph)
+  cudaGraphExec_t gfork[2] = {nullptr, nullptr};
+  int fork_kernels[2] = {0, 0};
+  long gen_steps = 0;  // graph steps of this generation
   // per-kernel event timing (gd_profile_enable)
   bool profiling = false;
   struct ProfRec { const char* name; cudaEvent_t a, b; };
