@@ -21,7 +21,11 @@ namespace {
 // State fields of the configuration: the five of the reference's step, and
 // composition when configured.
 // Largest four-component Fourier buffer of a model whose captured step runs its
-// phases side by side (step_sequence_forked); above, the kernels fill the chip.
+// phases side by side (step_sequence_forked), which needs twice as much again.  A
+// step, chain -> side by side, us (B200): 0.3 MiB (lmax 15, nr 12) 105 -> 58; 3 MiB
+// (31, 32) 144 -> 91; 12 MiB (63, 33) 243 -> 172; 24 MiB (63, 65) 336 -> 276; 48 MiB
+// (63, 129) 552 -> 500; 63 MiB (127, 42) 700 -> 634: the gain falls with the size,
+// as the kernels fill the chip, while the memory grows.
 constexpr size_t FORK_BYTES = (size_t)64 << 20;
 // Steps with the same settings after which they do.  Capturing and destroying the
 // two graphs with branches costs 1.3 ms beyond the chain's, the saving of 15 to 30
@@ -299,13 +303,7 @@ int setup(gd_handle* h) {
   AL(h->d_cbvals, 2 * NL); AL(h->d_csources, NR); AL(h->d_bctype, 4 * NL); AL(h->d_tau, 4 * NR);
   AL(h->d_tauc, 6 * (size_t)d.nseg);
   AL(h->d_grid, NGRID * h->grid_elems());
-  {
-    // with room for the phases of a captured step side by side where they run so
-    const size_t comp = NR * (d.M + 1) * d.nlat;
-    const bool more = c.precision == GD_PREC_FP64 && c.magnetic && !c.composition && 4 * comp * sizeof(double2) <= FORK_BYTES;
-    AL(h->d_F, (more ? 12 : 4) * comp);
-    if (more) h->d_F2 = h->d_F + 4 * comp;
-  }
+  AL(h->d_F, 4 * NR * (d.M + 1) * d.nlat);
   AL(h->d_epart, 2 * GD_ENERGY_BLOCKS * d.nseg); AL(h->d_eout, 2 * d.nseg);
 
   cudaStream_t s = h->stream;
@@ -775,8 +773,7 @@ int step_sequence(gd_handle* h, int boot) {
 // ones are written after them; the velocity products read j and B of the step
 // before, the induction the new velocity.  The kernels and their inputs are those
 // of step_sequence, so are the results, to the last bit.
-// Measured (B200, us a step, chain -> side by side): lmax 31, nr 32 CNAB2: 155 ->
-// 99; lmax 63, nr 65 EAB2, with loading and reading the state: 463 -> 396.
+// Times on both sides: FORK_BYTES.
 bool can_fork(const gd_handle* h) {
   const size_t comp = (size_t)h->d.nr * (h->d.M + 1) * h->d.nlat * sizeof(double2);
   return h->precision == GD_PREC_FP64 && !h->ext_derivs && h->c.magnetic && !h->c.composition && 4 * comp <= FORK_BYTES;
@@ -806,7 +803,7 @@ int step_sequence_forked(gd_handle* h, int boot) {
   const Dims& d = h->d;
   const cudaStream_t s = h->stream;
   const size_t comp = (size_t)d.nr * (d.M + 1) * d.nlat, G = h->grid_elems();
-  double2 *const Fv = h->d_F2, *const Fm = h->d_F2 + 4 * comp;
+  double2 *const Fv = h->d_F2, *const Fm = h->d_F2 + 4 * comp;  // fork_buffer
   CaptureBranches br{s};
   auto synth = [&](const double* tor, const double* pol, double2* F) {
     SynthArgs a{};
@@ -930,6 +927,24 @@ int capture_step(gd_handle* h, int boot, bool forked, cudaGraphExec_t* ge, int* 
   return GD_OK;
 }
 
+// The Fourier components of the velocity and the magnetic phase beside d_F's, made
+// when the branches first take over (a handle that only transforms, or steps in an
+// ensemble's graph, needs none); without memory for them the handle keeps the chain.
+bool fork_buffer(gd_handle* h) {
+  if (h->d_F2 || h->no_fork) return h->d_F2 != nullptr;
+  // an allocation now, in the middle of a run, must not disturb a capture on another thread
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  const bool swapped = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+  const std::string err = h->err;
+  h->no_fork = dalloc(h, &h->d_F2, (size_t)8 * h->d.nr * (h->d.M + 1) * h->d.nlat) != GD_OK;
+  if (h->no_fork) {
+    cudaGetLastError();
+    h->err = err;
+  }
+  if (swapped) cudaThreadExchangeStreamCaptureMode(&mode);
+  return !h->no_fork;
+}
+
 // The step graph for the current nonlinear bank and bootstrap flag: the chain, and
 // for small FP64 models the side-by-side form once FORK_AFTER steps have run with
 // the same settings.  Measured (B200, lmax 31, nr 32): capture and instantiation
@@ -938,7 +953,7 @@ int capture_step(gd_handle* h, int boot, bool forked, cudaGraphExec_t* ge, int* 
 int ensure_graph(gd_handle* h, int boot, cudaGraphExec_t* ge, int* kernels = nullptr) {
   const int p = h->nl_par;
   // (a bootstrap step between others, as after restoring a start, takes the chain)
-  const bool forked = h->gen_steps >= FORK_AFTER && boot == h->c.ab_mode && h->d_F2 && can_fork(h);
+  const bool forked = h->gen_steps >= FORK_AFTER && boot == h->c.ab_mode && can_fork(h) && fork_buffer(h);
   cudaGraphExec_t& held = forked ? h->gfork[p] : h->gexec[p][boot];
   int& count = forked ? h->fork_kernels[p] : h->graph_kernels[p][boot];
   if (!held) {

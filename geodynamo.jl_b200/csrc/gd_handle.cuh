@@ -88,8 +88,9 @@ struct gd_handle {
   double* d_grid = nullptr;   // NGRID grids (FP64)
   double2* d_F = nullptr;     // Fourier buffer, 4 components
   // captured steps of small FP64 models run their phases side by side
-  // (step_sequence_forked): eight more Fourier components (null: none)
+  // (step_sequence_forked): eight more Fourier components (lazy; no_fork: no memory for them)
   double2* d_F2 = nullptr;
+  bool no_fork = false;
   double *d_epart = nullptr, *d_eout = nullptr;
   // host-ABI staging (lazy)
   double *d_stage_spec = nullptr, *d_stage_spec2 = nullptr, *d_stage_grid = nullptr, *d_stage_grid2 = nullptr;

@@ -84,3 +84,20 @@ def test_restored_start_bootstraps_again(gdb):
     for x, y in zip(*out):
         assert np.array_equal(x, y, equal_nan=True)
     g.close()
+
+
+def test_memory_of_the_branches_comes_with_them(gdb):
+    lmax, nlat, nlon, nr = 31, 48, 96, 32
+    g = _model(gdb, lmax, nlat, nlon, nr, bc_mode=2)
+    h = gdb.SHTnsKitConfig(lmax, nlat, nlon, nr, dt=1e-6, bc_mode=2, composition=1)  # composition: always the chain
+    components = 16 * nr * (lmax + 1) * nlat
+    h.step(1)
+    g.step(AFTER)
+    before, other = g.device_bytes(), h.device_bytes()
+    g.step(1)
+    h.step(AFTER + 1)
+    assert g.device_bytes() == before + 8 * components and h.device_bytes() == other
+    g.step(4)
+    assert g.device_bytes() == before + 8 * components
+    g.close()
+    h.close()
