@@ -1250,14 +1250,18 @@ static int temperature_pullback_impl(gd_handle* h, const double* lam_re, const d
     return st;
   };
   auto usolve = [&](const double* x, double* y) { return cnab2_adjoint(h, GD_U_TOR, 2, 0, x, y); };  // D S^-T C
+  auto zero = [&](double* x, size_t n) {
+    const cudaError_t e = cudaMemsetAsync(x, 0, n * sizeof(double), h->stream);
+    return e == cudaSuccess ? GD_OK : fail(h, GD_ERR_CUDA, std::string("pullback scratch: ") + cudaGetErrorString(e));
+  };
   h->hold_sync = true;
   int s = gd_spectral_device(h, const_cast<double*>(lam_re), const_cast<double*>(lam_im), lam, 1);
   if (s) return done(s);
   s = gd_cnab2_adjoint(h, GD_TEMP, 0, lam, psi1);
   if (s) return done(s);
-  cudaMemsetAsync(psi2, 0, se * sizeof(double), h->stream);
+  s = zero(psi2, se);
   // the velocity after the run carries no cotangent of its own here
-  if (vel) cudaMemsetAsync(ul, 0, 12 * se * sizeof(double), h->stream);
+  if (s == GD_OK && vel) s = zero(ul, 12 * se);
   for (int k = nseg - 1; k >= 0 && s == GD_OK; --k) {
     const int c0 = k * C, c1 = std::min(K, c0 + C);
     s = gd_snapshot(h, h->t_snaps[k], 1);
@@ -1286,7 +1290,7 @@ static int temperature_pullback_impl(gd_handle* h, const double* lam_re, const d
         if (s == GD_OK) launch_axpby(h->stream, 2 * se, 1.0, ul, 1.0, unlt, ul);
         if (s == GD_OK) launch_axpby(h->stream, 2 * se, 1.0, ul, 1.0, usrc, ul);
         if (s == GD_OK && n >= 1) s = gd_temperature_u_adjoint(h, u + 2 * G, u + 3 * G, tmp, usrc);
-        if (s == GD_OK && n == 0) cudaMemsetAsync(usrc, 0, 2 * se * sizeof(double), h->stream);
+        if (s == GD_OK && n == 0) s = zero(usrc, 2 * se);
       }
       if (s == GD_OK && n > 0) {
         std::swap(psi1, psi2);
