@@ -254,9 +254,10 @@ __global__ void __launch_bounds__(128, 3) k_cnab2(Dims d, const int* __restrict_
 // substitution.  Rows come in batches whose loads are issued one batch ahead.
 //
 // What bounds it: load latency (a row of a column is 64 bytes of fields and 80
-// of factors, and its substitution waits for the row before).  The sweeps below
-// spent ~600 instructions a row: windows shifted by moves, factor addresses in
-// 64 bits, two divisions.  Here nine rows are unrolled per round, so a window
+// of factors, and its substitution waits for the row before).  The single sweeps
+// above execute about 470 warp instructions a row (ncu, 79.4 M for 5 x 32896
+// columns of 33 rows): they shift their windows, test every column, form 64-bit
+// factor offsets and divide.  Here nine rows are unrolled per round, so a window
 // index is a constant; factors come as 16-byte loads at 32-bit offsets from
 // uniform bases; no column is tested (tables and windows are zero outside the
 // matrix); the stored reciprocal with one correction step (quotient()) stands for

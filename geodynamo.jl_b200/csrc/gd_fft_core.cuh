@@ -190,8 +190,8 @@ __device__ typename C2<RT>::T* fft_forward(typename C2<RT>::T* a, typename C2<RT
 
 // ---------------------------------------------------------------------------
 // Compile-time variants for the transform lengths in use: every index
-// division below is by a constant (the runtime-plan kernels above spend most
-// of their instructions in integer division).
+// division below is by a constant (the runtime-plan kernels above divide by
+// run-time values for every element).
 // ---------------------------------------------------------------------------
 struct CPlan {
   int n, ns;

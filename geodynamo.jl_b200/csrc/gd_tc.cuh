@@ -44,9 +44,9 @@ __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
-// One lane of a converged warp.  A branch on it (unlike lane == 0) leaves the
-// operands of the tensor-core instructions in uniform registers, where they
-// are read from; they were moved there one by one for every instruction.
+// One lane of a converged warp.  elect.sync names the same lane each time for the
+// same mask (PTX ISA), so MMAs and the commits that cover them, all issued under
+// it, come from one thread.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}\n" : "=r"(p));
