@@ -237,61 +237,38 @@ template <typename RT, int N> struct CtGeom {
   static constexpr int MINB = 768 / NT;  // blocks per SM: 24 warps at 80 registers a thread
 };
 
-// One compile-time Stockham pass.  Padded indices pidx(j + r * stride) are
-// formed as pidx(j) + r * (stride + stride / 16) when the stride is a multiple
-// of 16 (and as pidx(group base) + offset when a radix group cannot cross a
-// 16-element boundary), so the inner loops carry no index arithmetic.  tw is
-// this pass's own table [r - 1][k] (k < NS, consecutive k in consecutive entries,
-// so a warp's twiddle reads are conflict-free in shared memory).
-template <int R, int N, int TB, int NS, typename C, int NT, bool XS>
+// One compile-time Stockham pass between two buffers of rows in the unpadded xidx
+// layout.  tw is this pass's own table [r - 1][k] (k < NS, consecutive k in
+// consecutive entries, so a warp's twiddle reads are conflict-free in shared memory).
+template <int R, int N, int TB, int NS, typename C, int NT>
 __device__ __forceinline__ void ct_pass(const C* __restrict__ src, C* __restrict__ dst, const C* __restrict__ tw) {
-  constexpr int RS = XS ? N : (N + (N >> 4)) | 1;
   constexpr int NBF = N / R;
   constexpr int TOTAL = TB * NBF;
   for (int b = threadIdx.x; b < TOTAL; b += NT) {
     const int row = b / NBF, j = b - row * NBF;
     const int k = j % NS;
-    const C* s = src + row * RS;
+    const C* s = src + row * N;
     C v[R];
-    if constexpr (XS) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = s[xidx(j + r * NBF)];
-    } else if constexpr (NBF % 16 == 0) {
-      const C* sj = s + pidx(j);
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = sj[r * (NBF + NBF / 16)];
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = s[pidx(j + r * NBF)];
-    }
+    for (int r = 0; r < R; ++r) v[r] = s[xidx(j + r * NBF)];
     if constexpr (NS > 1) {
 #pragma unroll
       for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw[(r - 1) * NS + k]);
     }
     Dft<R, C>::run(v);
-    C* o = dst + row * RS;
-    const int base = (j / NS) * NS * R;
-    const int o0 = base + k;
-    if constexpr (XS) {
+    C* o = dst + row * N;
+    const int o0 = (j / NS) * NS * R + k;
 #pragma unroll
-      for (int r = 0; r < R; ++r) o[xidx(o0 + r * NS)] = v[r];
-    } else if constexpr (NS % 16 == 0) {
-      C* oo = o + pidx(o0);
-#pragma unroll
-      for (int r = 0; r < R; ++r) oo[r * (NS + NS / 16)] = v[r];
-    } else if constexpr (16 % (NS * R) == 0) {
-      C* oo = o + o0 + (base >> 4);
-#pragma unroll
-      for (int r = 0; r < R; ++r) oo[r * NS] = v[r];
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) o[pidx(o0 + r * NS)] = v[r];
-    }
+    for (int r = 0; r < R; ++r) o[xidx(o0 + r * NS)] = v[r];
   }
 }
 
 // One compile-time pass within one buffer: every thread takes its butterflies'
 // inputs into registers, and after a barrier the results go back to the buffer.
+// Padded indices pidx(j + r * stride) are formed as pidx(j) + r * (stride +
+// stride / 16) when the stride is a multiple of 16 (and as pidx(group base) +
+// offset when a radix group cannot cross a 16-element boundary), so the inner loops
+// carry no index arithmetic.
 // INS: inputs from the buffer, else ld(row, index); OUTS: st(row, index, value)
 // goes to the buffer, else st itself takes the value (a consumer that is
 // pointwise in the output index).  tw: the passes' roots (make_twiddles), this
@@ -377,27 +354,17 @@ __device__ __forceinline__ void ct_run(C* buf, const C* __restrict__ tw, L& ld, 
 // A compile-time pass that hands its outputs (row, natural index, value) to
 // f instead of storing them: the last pass of a transform whose consumer is
 // pointwise in the output index.
-template <int R, int N, int TB, int NS, typename C, int NT, bool XS, class F>
+template <int R, int N, int TB, int NS, typename C, int NT, class F>
 __device__ __forceinline__ void ct_pass_apply(const C* __restrict__ src, const C* __restrict__ tw, F& f) {
-  constexpr int RS = XS ? N : (N + (N >> 4)) | 1;
   constexpr int NBF = N / R;
   constexpr int TOTAL = TB * NBF;
   for (int b = threadIdx.x; b < TOTAL; b += NT) {
     const int row = b / NBF, j = b - row * NBF;
     const int k = j % NS;
-    const C* s = src + row * RS;
+    const C* s = src + row * N;
     C v[R];
-    if constexpr (XS) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = s[xidx(j + r * NBF)];
-    } else if constexpr (NBF % 16 == 0) {
-      const C* sj = s + pidx(j);
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = sj[r * (NBF + NBF / 16)];
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = s[pidx(j + r * NBF)];
-    }
+    for (int r = 0; r < R; ++r) v[r] = s[xidx(j + r * NBF)];
     if constexpr (NS > 1) {
 #pragma unroll
       for (int r = 1; r < R; ++r) v[r] = cmul(v[r], tw[(r - 1) * NS + k]);
@@ -442,31 +409,18 @@ __device__ __forceinline__ void ct_fill_pass_twiddles(const float2* __restrict__
   }
 }
 
-// All passes between two buffers (tables: ct_fill_pass_twiddles); XS: rows in the unpadded xidx layout.
-template <int N, int TB, int S, int NS, typename C, int NT, int OFF = 0, bool XS = false>
-__device__ __forceinline__ C* ct_passes_pt(C* src, C* dst, const C* tw) {
-  constexpr CPlan P = PlanOf<N>::p;
-  if constexpr (S >= P.ns) {
-    return src;
-  } else {
-    constexpr int R = P.r[S];
-    ct_pass<R, N, TB, NS, C, NT, XS>(src, dst, tw + OFF);
-    __syncthreads();
-    return ct_passes_pt<N, TB, S + 1, NS * R, C, NT, (NS > 1 ? OFF + (R - 1) * NS : OFF), XS>(dst, src, tw);
-  }
-}
-
-// ct_passes_pt whose last pass hands its outputs to f (ct_pass_apply).
-template <int N, int TB, int S, int NS, typename C, int NT, int OFF, bool XS, class F>
-__device__ __forceinline__ void ct_passes_pt_apply(C* src, C* dst, const C* tw, F& f) {
+// All passes between two buffers (tables: ct_fill_pass_twiddles), the last one
+// handing its outputs to f (ct_pass_apply).
+template <int N, int TB, int S, int NS, typename C, int NT, int OFF, class F>
+__device__ __forceinline__ void ct_passes_apply(C* src, C* dst, const C* tw, F& f) {
   constexpr CPlan P = PlanOf<N>::p;
   constexpr int R = P.r[S];
   if constexpr (S == P.ns - 1) {
-    ct_pass_apply<R, N, TB, NS, C, NT, XS>(src, tw + OFF, f);
+    ct_pass_apply<R, N, TB, NS, C, NT>(src, tw + OFF, f);
   } else {
-    ct_pass<R, N, TB, NS, C, NT, XS>(src, dst, tw + OFF);
+    ct_pass<R, N, TB, NS, C, NT>(src, dst, tw + OFF);
     __syncthreads();
-    ct_passes_pt_apply<N, TB, S + 1, NS * R, C, NT, (NS > 1 ? OFF + (R - 1) * NS : OFF), XS>(dst, src, tw, f);
+    ct_passes_apply<N, TB, S + 1, NS * R, C, NT, (NS > 1 ? OFF + (R - 1) * NS : OFF)>(dst, src, tw, f);
   }
 }
 

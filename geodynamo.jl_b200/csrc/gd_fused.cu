@@ -1,10 +1,12 @@
 // gd_fused.cu -- the grid-space part of each nonlinear phase of the
-// mixed-precision step in one kernel, for any row length (the lengths of
-// gd_fused_reg.cuh have a register-resident form of the phases with products): inverse phi transforms of the phase's
+// mixed-precision step in one kernel: inverse phi transforms of the phase's
 // synthesized components, the pointwise products, and the forward phi
 // transform with the Gauss-weighted north/south folds that the Legendre
 // analysis consumes.  The physical grids of a phase live only in shared
 // memory; HBM sees the Fourier coefficients in and the folded transforms out.
+// The phases run here at row lengths without a register-resident form
+// (gd_fused_reg.cuh), by a plan at run time; grids on request run here at every
+// length, the 3/2-rule ones by plans at compile time.
 //
 // CTA = (block of FOURIER_BLOCK north/south colatitude pairs, shell).  The
 // Fourier input is the blocked layout written by the tensor-core synthesis:
@@ -46,15 +48,6 @@ __host__ __device__ __forceinline__ int row_stride(int n) {
   else return prow(n);
 }
 
-template <int N>
-__device__ __forceinline__ float2* run_fft(float2* a, float2* b, const float2* tw, const FftPlan& p) {
-  if constexpr (N > 0) {
-    return ct_passes_pt<N, FB, 0, 1, float2, FNT, 0, true>(a, b, tw);
-  } else {
-    return fft_forward<float, FNT>(a, b, FB, p, tw);
-  }
-}
-
 // Z_m = F_N + i F_S and Z_{n-m} = conj(F_N) + i conj(F_S), stored conjugated
 // (the inverse transform is conj(FFT(conj(Z)))): element e = m * FB + pair.
 template <int N>
@@ -74,11 +67,8 @@ __device__ __forceinline__ void pack_z(float2* bufA, int rs, int n, int e, int r
 // < P, the conjugated input y is zero on P <= k <= 2P, so with phi = 3 c + a
 // the inverse transform is three P-point transforms of
 //   W_a[k] = W^(k a) (y_k + y_(k + 2P) W^(2 P a)),   W = exp(-2 pi i / n),
-// built straight from the frequency pair (k, P - k) -- no zero band and no
-// radix-3 pass -- and the forward transform's outputs X_m, X_(n - m) (m <= M)
-// follow from the P-point transforms Y_a of the sub-rows x_(3 c + a):
-//   X_m = sum_a W^(m a) Y_a[m],  X_(n - m) = sum_a W^(-m a) Y_a[(P - m) mod P].
-// Sub-row (pair ii, a) holds P elements at (3 ii + a) P in the xidx layout.
+// built straight from the frequency pair (k, P - k): no zero band and no
+// radix-3 pass.  Sub-row (pair ii, a) holds P elements at (3 ii + a) P in the xidx layout.
 template <int N> struct Split3 {
   static constexpr int P = N / 3;
   static constexpr bool ok = N > 0 && N % 3 == 0 && P >= 8 && (P & (P - 1)) == 0;
@@ -90,6 +80,7 @@ __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.
 
 template <int N, int PH, bool S3>
 __global__ void __launch_bounds__(FNT, 4) k_fused(Dims d, FftPlan p, const float2* __restrict__ tw, FusedArgs a) {
+  static_assert(N == 0 || PH == FUSED_GRID, "the products' compile-time lengths are those of gd_fused_reg.cuh");
   typedef float2 C;
   constexpr int P = S3 ? N / 3 : 1;
   const int n = N > 0 ? N : p.n;
@@ -298,12 +289,12 @@ __global__ void __launch_bounds__(FNT, 4) k_fused(Dims d, FftPlan p, const float
     __syncthreads();
     if (c + 1 < a.nin) prefetch(c + 1);
     if constexpr (S3) {
-      ct_passes_pt_apply<P, 3 * FB, 0, 1, C, FNT, 0, true>(bufA, bufB, stw, consume_s3);
+      ct_passes_apply<P, 3 * FB, 0, 1, C, FNT, 0>(bufA, bufB, stw, consume_s3);
     } else if constexpr (N > 0) {
       // the last Stockham pass feeds the consumer directly
-      ct_passes_pt_apply<N, FB, 0, 1, C, FNT, 0, true>(bufA, bufB, stw, consume_n);
+      ct_passes_apply<N, FB, 0, 1, C, FNT, 0>(bufA, bufB, stw, consume_n);
     } else {
-      const C* res = run_fft<N>(bufA, bufB, stw, p);
+      const C* res = fft_forward<float, FNT>(bufA, bufB, FB, p, stw);
       for (int e = tid; e < FB * n; e += FNT) {
         const int ii = e / n, j = e - ii * n;
         consume_n(ii, j, res[ii * rs + ridx<N>(j)]);
@@ -317,27 +308,15 @@ __global__ void __launch_bounds__(FNT, 4) k_fused(Dims d, FftPlan p, const float
   const float sc = (float)(2.0 * 3.14159265358979323846 / n);
   const int nout = (PH == FUSED_TEMPERATURE) ? 1 : 2;
   for (int o = 0; o < nout; ++o) {
-    C* src = o == 0 ? acc0 : acc1;
-    const C* res;
-    if constexpr (S3) res = ct_passes_pt<P, 3 * FB, 0, 1, C, FNT, 0, true>(src, o == 0 ? bufA : bufB, stw);
-    else res = run_fft<N>(src, o == 0 ? bufA : bufB, stw, p);
+    const C* res = fft_forward<float, FNT>(o == 0 ? acc0 : acc1, o == 0 ? bufA : bufB, FB, p, stw);
     const size_t gb = ((size_t)(o * d.nr + r) * (M + 1)) * 2 * d.nth;
     for (int e = tid; e < tot; e += FNT) {
       const int m = e / FB, ii = e - m * FB;
       if (ii >= rows) continue;
       const int ith = i0 + ii;
-      C zk, zn;
-      if constexpr (S3) {
-        const C* y = res + ii * N;  // Y_a at y + a P
-        const int xm = xidx(m), xp = xidx(m == 0 ? 0 : P - m);
-        const C w1 = stw3[m], w2 = stw3[2 * m];
-        zk = cadd(y[xm], cadd(cmul(w1, y[P + xm]), cmul(w2, y[2 * P + xm])));
-        zn = cadd(y[xp], cadd(cmul(conjf2(w1), y[P + xp]), cmul(conjf2(w2), y[2 * P + xp])));
-      } else {
-        const C* row = res + ii * rs;
-        zk = row[ridx<N>(m)];
-        zn = row[ridx<N>(m == 0 ? 0 : n - m)];
-      }
+      const C* row = res + ii * rs;
+      const C zk = row[pidx(m)];
+      C zn = row[pidx(m == 0 ? 0 : n - m)];
       zn.y = -zn.y;
       const float Xx = 0.5f * (zk.x + zn.x), Xy = 0.5f * (zk.y + zn.y);
       const float Yx = 0.5f * (zk.y - zn.y), Yy = -0.5f * (zk.x - zn.x);
@@ -400,8 +379,6 @@ bool launch_fused_len7(cudaStream_t s, const Dims& d, int nlon, const void* tw, 
 int fourier_blocks(const Dims& d) { return ceil_div(d.nth, FB); }
 
 size_t fourier_comp_elems(const Dims& d) { return (size_t)d.nr * fourier_blocks(d) * (d.M + 1) * FB; }
-
-size_t fused_smem_bytes(int phase, int nlon) { return fused_smem(phase, nlon, false); }
 
 void launch_fused(cudaStream_t s, const Dims& d, const FftPlan& p, const void* twf, int phase, const FusedArgs& a) {
   const float2* tw = static_cast<const float2*>(twf);

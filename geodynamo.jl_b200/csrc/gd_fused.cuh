@@ -24,7 +24,6 @@ struct FusedArgs {
 // Theta blocks of the blocked Fourier layout and float4 elements per component.
 int fourier_blocks(const Dims& d);
 size_t fourier_comp_elems(const Dims& d);
-size_t fused_smem_bytes(int phase, int nlon);
 void launch_fused(cudaStream_t s, const Dims& d, const FftPlan& p, const void* twf, int phase, const FusedArgs& a);
 
 }  // namespace gd
