@@ -892,11 +892,15 @@ def main():
             if len(bounds) > 1:
                 roofline["other"] = {k: bounds[1][k] for k in ("bound", "achieved", "peak", "unit", "frac")}
             if top["name"].startswith("fused_"):
-                # what does bind the fused phase kernels (one-launch ncu capture at nr = 33,
+                # what does bind the fused phase kernels (one-launch ncu captures at nr = 33 of nlon 768,
                 # profiles/phase_kernels_shell_l255_nr33_mixed_vel64.md): neither HBM nor a tensor pipe
-                roofline["binding_unit"] = {"unit": "shared-memory (LSU) wavefronts and issue at two warps a scheduler",
-                                            "lsu_frac": 0.46, "issue_active_frac": 0.48,
-                                            "source": "ncu, k_fused_reg<RowPlan<16, 3, 16>, true, 2>, shell_l255_nr33"}
+                captured = {"temperature": (1, 0.47, 0.44), "velocity": (2, 0.46, 0.48), "induction": (3, 0.47, 0.45)}
+                phase = captured.get(top["name"].split("_")[1])
+                if phase and p["nlon"] == 768:
+                    roofline["binding_unit"] = {"unit": "shared-memory (LSU) wavefronts and issue at two warps a scheduler",
+                                                "lsu_frac": phase[1], "issue_active_frac": phase[2],
+                                                "source": "ncu, k_fused_reg<RowPlan<16, 3, 16>, true, %d>, "
+                                                          "shell_l255_nr33" % phase[0]}
 
     # ---- FP64 reference step on the GPU (denominator of the metric) ----
     fp64_value = None

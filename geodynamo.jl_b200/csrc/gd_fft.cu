@@ -333,9 +333,12 @@ k_coriolis_fused(Dims d, const double2* __restrict__ tw,
   }
 }
 
-// Lengths with FP64 kernels of their own: products of 2, 3 and 5 near the grids of
-// truncations up to 341, the fused phases' lengths.  Other lengths run the plan at
-// run time, whose index divisions and two buffers cost 10 to 45 % of a step (33
+// Lengths with FP64 kernels of their own: the 32 that have a register plan for the
+// FP32 phases (gd_fused_len*.cu), so that the precisions of a model change kernels
+// at the same lengths.  They are a choice among the products of 2, 3 and 5 up to 1024,
+// not all that the grid rules give: 54, 60, 72, 90, 120, 150, 240, 250, 270, 480, 540, 864
+// and others are not built (each adds 2 MB of kernels to the library) and run the
+// plan at run time, whose index divisions and two buffers cost 10 to 45 % of a step (33
 // shells, us, plan at run time -> its own kernels; FP64 / velocity chain in FP64):
 // nlon 64 90 -> 83 / 169 -> 159; 256 349 -> 252 / 326 -> 282; 512 1665 -> 1125 /
 // 876 -> 698; 900 5350 -> 3261 / 2724 -> 2120; faster at every length listed.

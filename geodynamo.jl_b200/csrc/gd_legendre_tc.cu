@@ -6,9 +6,10 @@
 // every tile product is hi*hi + hi*lo + lo*hi, which carries about 22 bits.
 // The associated Legendre tables (Pbar, dPbar/dtheta, m Pbar / sin) are stored
 // once as pre-split, pre-swizzled shared-memory images (K-major SWIZZLE_128B
-// tiles of 128 rows x 32 TF32); the runtime operand (spectral coefficients for
-// synthesis, folded phi transforms for analysis) is split by the loader
-// threads while it is written to shared memory.
+// tiles of 128 rows x 32 TF32).  The runtime operand is split on its way in: the
+// spectral coefficients of the synthesis arrive as FP32 chunks that converter warps
+// split in place, the folded phi transforms of the analysis are split by its loader
+// threads while they are written to shared memory.
 //
 // Parity: for each order m the sum over l splits by the parity of l - m.
 // Synthesis keeps the even and odd partial sums in separate tensor-memory
@@ -36,9 +37,10 @@ constexpr int TC_N2 = 128;    // synthesis and scalar analysis column tile
 constexpr int TC_K = 32;                       // TF32 elements per 128-byte row
 constexpr int TILE_A_FLOATS = TC_M * TC_K;      // 4096 floats = 16 KB
 constexpr int CHUNK_FLOATS = 2 * TILE_A_FLOATS; // hi image then lo image (32 KB)
-// Pipelined kernels: every stage holds one (chunk, parity) step; stages sit
-// back to back after a 1024-byte aligned base, then one mbarrier per stage
-// and the TMEM address slot (192 KB + alignment slack per CTA).
+// Both kernels keep their slots back to back after a 1024-byte aligned base, then the
+// mbarriers and the TMEM address slot: the synthesis two rings of 32 KB slots, seven
+// in all (six in the scalar form), the analysis two stages of one (chunk, parity or
+// fold) step each, 192 KB in the vector and 128 KB in the scalar form.
 
 __device__ __forceinline__ int kpar(int L, int m, int p) { return p == 0 ? (L - m + 2) / 2 : (L - m + 1) / 2; }
 __device__ __host__ __forceinline__ int nck_h(int L, int m, int p) {
@@ -306,7 +308,7 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_tc_synth4(Dims d, const int* 
                                                              const double* __restrict__ sinv, TcSynthArgs a, int ntt,
                                                              int ncol) {
   constexpr int NCS = VEC ? TC_N2 : 2 * TC_N2;   // columns per tile: vector 128, scalar 256
-  constexpr int BT = NCS * TC_K;                  // one B image (hi or lo)
+  constexpr int BT = NCS * TC_K;                  // one FP32 coefficient chunk
   constexpr uint32_t NCOL = 512;
   extern __shared__ unsigned char smem_raw[];
   const uintptr_t base = (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023);
@@ -919,12 +921,11 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_tc_analysis3(Dims d, const in
 }
 
 // ---------------------------------------------------------------------------
-// Synthesis: stages + full/empty per stage, tfull, tempty, drain and the TMEM
-// address slot.  Analysis: stages + full/empty per stage, drain, the TMEM
+// Synthesis: slots (the vector form's seven) + full / empty of both rings and the raw
+// chunks, tfull, tempty, drain and the TMEM address slot.  Analysis: stages + full/empty per stage, drain, the TMEM
 // address slot and the scalar kernels' per-column tables (one pointer per
 // column, one offset per pair).
-static size_t synth_smem(bool vec) {
-  (void)vec;
+static size_t synth_smem() {
   return 1024 + (size_t)(SY_HMAX + SY_S) * SY_SLOT * 4 + 8 * (3 * SY_HMAX + 2 * SY_S + 4);
 }
 static size_t analysis_smem(bool vec) {
@@ -933,8 +934,8 @@ static size_t analysis_smem(bool vec) {
   return 1024 + (size_t)S * (A + B) * 4 + 8 * (2 * S + 2) + (size_t)NC * 8 + (size_t)(NC / 2) * 8;
 }
 static void set_attrs() {
-  allow_dynamic_smem(k_tc_synth4<false>, synth_smem(false));
-  allow_dynamic_smem(k_tc_synth4<true>, synth_smem(true));
+  allow_dynamic_smem(k_tc_synth4<false>, synth_smem());
+  allow_dynamic_smem(k_tc_synth4<true>, synth_smem());
   allow_dynamic_smem(k_tc_analysis3<false>, analysis_smem(false));
   allow_dynamic_smem(k_tc_analysis3<true>, analysis_smem(true));
 }
@@ -954,13 +955,13 @@ void launch_tc_synth(cudaStream_t s, const Dims& d, const int* moff, const long*
     const int ncol = ceil_div(a.nf * d.nr * 2, 2 * TC_N2);
     const int ntiles = (d.M + 1) * ntt * ncol;
     if (a.prep_mask) k_synth_coef_image<false><<<dim3(kcmax, d.M + 1, ncol), 256, 0, s>>>(d, moff, cofs, ntt, a);
-    k_tc_synth4<false><<<std::min(ntiles, cta_cap(a.max_ctas)), SY_THREADS, synth_smem(false), s>>>(d, moff, cofs, imgP,
+    k_tc_synth4<false><<<std::min(ntiles, cta_cap(a.max_ctas)), SY_THREADS, synth_smem(), s>>>(d, moff, cofs, imgP,
                                                                                           imgD, sinv, a, ntt, ncol);
   } else {
     const int ncol = ceil_div(d.nr, 32);
     const int ntiles = (d.M + 1) * ntt * ncol;
     if (a.prep_mask) k_synth_coef_image<true><<<dim3(kcmax, d.M + 1, ncol), 256, 0, s>>>(d, moff, cofs, ntt, a);
-    k_tc_synth4<true><<<std::min(ntiles, cta_cap(a.max_ctas)), SY_THREADS, synth_smem(true), s>>>(d, moff, cofs, imgP, imgD,
+    k_tc_synth4<true><<<std::min(ntiles, cta_cap(a.max_ctas)), SY_THREADS, synth_smem(), s>>>(d, moff, cofs, imgP, imgD,
                                                                                         sinv, a, ntt, ncol);
   }
 }

@@ -75,7 +75,7 @@ static size_t radial_smem() {
 // derivative i m, radial derivative by the banded D1, then x 1/r on the
 // angular components (:317-321).  In m-major order (l +- 1, m) sits at j +- 1.
 // IMG: the mixed path's scalar synthesis reads g_theta, g_phi, g_r as
-// TF32 image columns (field slots 1, 2, 3 of n = (field nr + r) 2 + re/im);
+// FP32 image columns (field slots 1, 2, 3 of n = (field nr + r) 2 + re/im);
 // they are written there instead of to the FP64 arrays.
 template <int KL, bool IMG>
 __global__ void k_gradients(Dims d, const int* __restrict__ lof, const int* __restrict__ mof,
