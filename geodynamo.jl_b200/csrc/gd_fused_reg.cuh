@@ -18,7 +18,7 @@
 // DFT fill 255 registers at N = 768) against shared-memory latency; issue ~45%,
 // FP32 pipe ~50%, shared memory ~50%.  Against radix passes of a whole CTA
 // through shared memory with the sums kept there (47 k warp instructions per
-// team and ten transforms, now 19 k) it has one exchange instead of three
+// team and ten transforms, now 17 k, ncu) it has one exchange instead of three
 // passes, no block barrier, no index arithmetic (every address is a thread base
 // plus a constant), no read-modify-write of the sums, and packed FP32 adds.
 // The exchange rows have an odd stride, so both its sides are free of bank
