@@ -2493,6 +2493,7 @@ int gd_ensemble_create(const gd_config* cfgs, int n, int device, gd_ensemble** o
       gd_ensemble_destroy(e);
       return s;
     }
+    h->in_ensemble = true;
     e->members.push_back(h);
     cudaEvent_t ev = nullptr;
     if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {

@@ -19,6 +19,7 @@ struct FusedArgs {
   const double* sources; // internal heat sources per shell
   float rf, lf;          // Pm/E for the advection and Lorentz factors
   float cf;              // Pm/E for the Coriolis term (0: the term is formed elsewhere)
+  bool dense;            // an ensemble's member: leave SMs to the other members' kernels
 };
 
 // Theta blocks of the blocked Fourier layout and float4 elements per component.

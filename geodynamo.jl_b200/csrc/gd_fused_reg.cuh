@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
   typedef float2 C;
   constexpr int T = PL::T, A = PL::A, B = PL::B, K = PL::K, N = PL::N, W = PL::W, TEAM = PL::TEAM, SB = PL::SB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x;
   int team, tl;  // team within the CTA, lane within the team
   unsigned mask = 0xffffffffu;
   if constexpr (TEAM <= 32) {
@@ -130,12 +130,12 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
   // tables shared by the CTA: W_N^(j u) at [u][j] (row stride T + 1), longitude factors of the Coriolis term
   C* const stw = reinterpret_cast<C*>(smem_raw);
   float* const sct = reinterpret_cast<float*>(stw + K * (T + 1));
-  for (int e = tid; e < K * T; e += 32 * G::WARPS) {
+  for (int e = tid; e < K * T; e += nt) {
     const int u = e / T, j = e - u * T;
     stw[u * (T + 1) + j] = tw[(u * j) % N];
   }
   if constexpr (PH == FUSED_VELOCITY) {
-    for (int e = tid; e < N; e += 32 * G::WARPS) sct[e] = (float)a.cth[e < d.nlat - 1 ? e : d.nlat - 1];
+    for (int e = tid; e < N; e += nt) sct[e] = (float)a.cth[e < d.nlat - 1 ? e : d.nlat - 1];
   }
   unsigned char* const mine = smem_raw + G::cta_bytes() + G::team_bytes() * team;
   float4* const sin_ = reinterpret_cast<float4*>(mine);
@@ -158,6 +158,10 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
   };
   const int j = tl >> 1, ii = tl & 1;
 
+  // Outputs of this CTA: all of the phase, or blockIdx.y of two; they take the
+  // components c0 .. c1 - 1 (a.fin: theta components, for the phi output 1, then phi components)
+  const bool apart = PH != FUSED_TEMPERATURE && gridDim.y == 2;
+  const int half = a.nin / 2, c0 = apart && blockIdx.y == 0 ? half : 0, c1 = apart && blockIdx.y == 1 ? half : a.nin;
   // input run of team index g and component c into stage st
   auto fetch = [&](int g, int c, int st) {
     const float4* src = a.fin[c] + (size_t)g * tot;
@@ -192,13 +196,13 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
 
   // Inverse transform of the staged component c; consume(base index, A q + a, z[T])
   // gets the T longitudes phi = A q + a + K p of each (a, w) as (north, -south).
-  auto inverse = [&](int c, int nin, auto&& consume) {
+  auto inverse = [&](int c, auto&& consume) {
     cp_async_wait<0>();
     sync();
     [[maybe_unused]] C y[G::HOLD ? (SPLIT ? 2 * B : K) : 1];
     auto next = [&](int stage) {
-      if (c + 1 < nin) fetch(gc, c + 1, stage);
-      else if (gn >= 0) fetch(gn, 0, stage);
+      if (c + 1 < c1) fetch(gc, c + 1, stage);
+      else if (gn >= 0) fetch(gn, c0, stage);
     };
     if constexpr (G::HOLD) {
       if constexpr (SPLIT) {
@@ -357,9 +361,9 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
   const float ur = 0.f, wr = 0.f, jr = 0.f, br = 0.f;
   // a warp's teams, and the warps of a team, run the same number of rounds;
   // a team past the last one repeats the last and stores nothing
-  const int first = blockIdx.x * G::TEAMS, stride = gridDim.x * G::TEAMS;
+  const int per_cta = G::teams_of(nt / 32), first = blockIdx.x * per_cta, stride = gridDim.x * per_cta;
   gn = min(first + team, nteams - 1);
-  fetch(gn, 0, 0);
+  fetch(gn, c0, 0);
   for (int base = first; base < nteams; base += stride) {
     gc = gn;
     const bool live = base + team < nteams;
@@ -370,7 +374,7 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
       const float s_r = (float)a.sources[r];
       C* const kp = keep + tl;
       for (int c = 0; c < 5; ++c) {
-        inverse(c, 5, [&](int e0, int, C* z) {
+        inverse(c, [&](int e0, int, C* z) {
           if (c == 0) {
 #pragma unroll
             for (int p = 0; p < T; ++p) acc[e0 + p] = make_float2(ur * z[p].x, ur * z[p].y);
@@ -395,11 +399,9 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
       //   theta: adv (u_ph w_r - u_r w_ph) + mrf (-ct u_ph) + lf (j_ph b_r - j_r b_ph)
       //   phi:   adv (u_r w_th - u_th w_r) + mrf (ct u_th + st u_r) + lf (j_r b_th - j_th b_r)
       // induction: u, b: theta u_ph b_r - u_r b_ph, phi u_r b_th - u_th b_r
-      // (a.fin: the theta components, then the phi components)
       const float rf_r = d.rfs32 ? d.rfs32[r] : a.rf;
       const float adv = -rf_r, mrf = a.cf != 0.f ? -rf_r : -a.cf, lfr = d.rfs32 ? rf_r : a.lf;
-      const int half = a.nin / 2;
-      for (int o = 1; o >= 0; --o) {
+      for (int o = c0 == 0; o >= (c1 == half); --o) {
         const float sg = o ? -1.f : 1.f;  // sign of the first term of each product pair
 #pragma unroll
         for (int e = 0; e < K; ++e) acc[e] = make_float2(0.f, 0.f);
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
           else kz = c == 0 ? adv * (sg * wr) : c == 1 ? adv * (-sg * ur) : c == 2 ? lfr * (sg * br) : lfr * (-sg * jr);
           const float2 kz2 = make_float2(kz, kz);
           const float kc = o ? mrf : -mrf;
-          inverse(o ? c : half + c, a.nin, [&](int e0, int ph0, C* z) {
+          inverse(o ? c : half + c, [&](int e0, int ph0, C* z) {
 #pragma unroll
             for (int p = 0; p < T; ++p) acc[e0 + p] = __ffma2_rn(kz2, z[p], acc[e0 + p]);
             if (PH == FUSED_VELOCITY && c == 0) {
@@ -431,10 +433,20 @@ template <class PL, bool SPLIT, int PH>
 void launch_fused_team(cudaStream_t s, const Dims& d, const float2* tw, const FusedArgs& a) {
   typedef FusedRegGeom<PL, SPLIT, PH> G;
   static_assert(G::smem() <= G::LIMIT, "shared memory");
-  const int nblk = fourier_blocks(d), nteams = nblk * d.nr;
-  const int ctas = ceil_div(nteams, G::TEAMS), most = current_sm_count() * G::MINB;
+  const int nblk = fourier_blocks(d), nteams = nblk * d.nr, sms = current_sm_count();
+  // A handle with the chip to itself whose teams do not give every SM a CTA: each
+  // output to CTAs of its own, and CTAs of just enough warps.  Packed into full CTAs a
+  // team took its outputs one after the other on a few SMs (velocity / temperature /
+  // induction phase at lmax 127, nlon 384, nr 9: 43 / 29 / 29 us, now 21 / 23 / 16;
+  // the passes of a whole CTA through shared memory took 27 / 18 / 17).
+  const bool spread = !a.dense && nteams < G::TEAMS * sms;
+  const int outputs = spread && PH != FUSED_TEMPERATURE ? 2 : 1;
+  int warps = spread ? PL::WPT : G::WARPS;
+  while (warps < G::WARPS && G::teams_of(warps) * sms < nteams * outputs) warps += PL::WPT;
+  const int teams = G::teams_of(warps), ctas = ceil_div(nteams, teams), most = sms * G::MINB;
   allow_dynamic_smem(k_fused_reg<PL, SPLIT, PH>, G::smem());
-  k_fused_reg<PL, SPLIT, PH><<<ctas < most ? ctas : most, 32 * G::WARPS, G::smem(), s>>>(d, tw, a, nblk, nteams);
+  k_fused_reg<PL, SPLIT, PH><<<dim3(ctas < most ? ctas : most, outputs), 32 * warps,
+                               G::cta_bytes() + G::team_bytes() * teams, s>>>(d, tw, a, nblk, nteams);
 }
 
 template <class PL, bool SPLIT>

@@ -27,6 +27,7 @@ struct gd_handle {
   // persistent CTAs of the tensor-core Legendre kernels (0: one per SM); an
   // ensemble caps them so that its members share the SMs
   int tc_ctas = 0;
+  bool in_ensemble = false;   // shares the chip with the ensemble's other members
   size_t bytes = 0;
   std::vector<void*> allocs;
 

@@ -211,6 +211,7 @@ FusedArgs phase_args(gd_handle* h) {
   f.rf = (float)(h->c.magnetic_prandtl / h->c.ekman);
   f.lf = f.rf;
   f.cf = f.rf;
+  f.dense = h->in_ensemble;
   return f;
 }
 
