@@ -434,13 +434,15 @@ void launch_fused_team(cudaStream_t s, const Dims& d, const float2* tw, const Fu
   typedef FusedRegGeom<PL, SPLIT, PH> G;
   static_assert(G::smem() <= G::LIMIT, "shared memory");
   const int nblk = fourier_blocks(d), nteams = nblk * d.nr, sms = current_sm_count();
-  // A handle with the chip to itself whose teams do not give every SM a CTA: each
-  // output to CTAs of its own, and CTAs of just enough warps.  Packed into full CTAs a
-  // team took its outputs one after the other on a few SMs (velocity / temperature /
-  // induction phase at lmax 127, nlon 384, nr 9: 43 / 29 / 29 us, now 21 / 23 / 16;
-  // the passes of a whole CTA through shared memory took 27 / 18 / 17).
+  // A handle with the chip to itself whose teams do not give every SM a full CTA: CTAs
+  // of just enough warps, and each output to CTAs of its own while those fit the SMs
+  // once (beyond, two rounds of one output take longer than one of both: lmax 47, nr
+  // 260 velocity 33 against 31 us).  Packed into full CTAs a team took its outputs one
+  // after the other on a few SMs (velocity / temperature / induction phase at lmax 127,
+  // nlon 384, nr 9: 43 / 29 / 29 us, now 21 / 23 / 16; the passes of a whole CTA through
+  // shared memory took 27 / 18 / 17).
   const bool spread = !a.dense && nteams < G::TEAMS * sms;
-  const int outputs = spread && PH != FUSED_TEMPERATURE ? 2 : 1;
+  const int outputs = spread && PH != FUSED_TEMPERATURE && 2 * nteams <= G::TEAMS * sms ? 2 : 1;
   int warps = spread ? PL::WPT : G::WARPS;
   while (warps < G::WARPS && G::teams_of(warps) * sms < nteams * outputs) warps += PL::WPT;
   const int teams = G::teams_of(warps), ctas = ceil_div(nteams, teams), most = sms * G::MINB;

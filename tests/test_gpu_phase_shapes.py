@@ -19,7 +19,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("lmax,nlat,nlon,nr,magnetic", [
     (7, 12, 24, 3, 1),        # fewer teams than SMs
     (31, 48, 96, 9, 0),       # two components an output
-    (31, 48, 96, 197, 1),     # 16 teams a CTA: the last nr that spreads
+    (31, 48, 96, 98, 1),      # 16 teams a CTA: the last nr with CTAs for each output
+    (31, 48, 96, 99, 1),
+    (31, 48, 96, 197, 1),     # and the last with fewer warps
     (31, 48, 96, 198, 1),
     (47, 50, 100, 20, 1),     # teams that do not fill a warp
     (63, 66, 128, 60, 1),
