@@ -460,7 +460,11 @@ void launch_fused_plan(cudaStream_t s, const Dims& d, const float2* tw, int phas
   }
 }
 
-// Row length N = T A B; A = 3 also in its SPLIT form when the orders allow it.
+// Row length N = T A B; A = 3 also in its SPLIT form when the orders allow it.  Where
+// the spectrum is not held (K > 40) a transform sums A points for each of A B values,
+// so such a length takes the split with the smaller A: 360 as 6 5 12 against 6 10 6,
+// velocity / temperature / induction phase at lmax 170, nr 33: 126 / 87 / 84 -> 84 / 60
+// / 56 us, nr 5: 126 / 84 / 83 -> 49 / 58 / 35 (plan at run time: 56 / 38 / 35).
 template <int T, int A, int B>
 bool launch_fused_row(cudaStream_t s, const Dims& d, const void* twf, int phase, const FusedArgs& a) {
   typedef RowPlan<T, A, B> PL;
