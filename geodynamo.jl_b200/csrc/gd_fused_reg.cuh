@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(32 * FusedRegGeom<PL, SPLIT, PH>::WARPS, Fused
   // Outputs of this CTA: all of the phase, or blockIdx.y of two; they take the
   // components c0 .. c1 - 1 (a.fin: theta components, for the phi output 1, then phi components)
   const bool apart = PH != FUSED_TEMPERATURE && gridDim.y == 2;
-  const int half = a.nin / 2, c0 = apart && blockIdx.y == 0 ? half : 0, c1 = apart && blockIdx.y == 1 ? half : a.nin;
+  const int nin = PH == FUSED_INDUCTION ? 4 : a.nin, half = nin / 2;
+  const int c0 = apart && blockIdx.y == 0 ? half : 0, c1 = apart && blockIdx.y == 1 ? half : nin;
   // input run of team index g and component c into stage st
   auto fetch = [&](int g, int c, int st) {
     const float4* src = a.fin[c] + (size_t)g * tot;
